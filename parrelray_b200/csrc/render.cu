@@ -194,9 +194,15 @@ prr_status build_plan(prr_ctx *ctx, const prr_frame_desc *frames, int n, RenderP
                 return bad(ctx, f, "sphere " + std::to_string(s) + " has a bad centre or radius");
             if (S.texture_id >= PRR_MAX_TEXTURES || (S.texture_id >= 0 && !ctx->tex[S.texture_id].buf.p))
                 return bad(ctx, f, "sphere " + std::to_string(s) + " texture id not uploaded");
-            // a hit with any window h <= hmax needs |p - c|^2 <= ((sqrt(hmax) + R)/2)^2 + R^2
-            double reach = 0.5 * (std::sqrt((double)d.hmax) + S.radius);
-            float far2 = (float)((reach * reach + (double)S.radius * S.radius) * 1.01 + 1e-3);
+            // a hit with any window w <= hmax needs |p - c|^2 <= ((sqrt(hmax) + R)/2)^2 + R^2, and also
+            // <= R^2 + hmax/3: with c = D^2 - R^2 > 0 and b = -v.(p - c), the test's distance d = 2b -
+            // sqrt(b^2 - c) is least at b^2 = 4c/3, where d = sqrt(3c), and a hit needs d^2 <= w.  (0.1 %
+            // covers the rounding of the test, which is relative to D^2; a first step h above hmax can open
+            // a wider window, so the second bound is for h <= hmax only.)
+            const double reach = 0.5 * (std::sqrt((double)d.hmax) + S.radius), R2 = (double)S.radius * S.radius;
+            double f2 = (reach * reach + R2) * 1.01 + 1e-3;
+            if (d.h <= d.hmax) f2 = std::min(f2, (R2 + d.hmax / 3.0) * 1.001);
+            const float far2 = (float)f2;
             p.sph[s] = {S.center[0], S.center[1], S.center[2], S.radius, dev_tex(ctx, S.texture_id), far2,
                         (float)std::sqrt((double)far2)};
         }
