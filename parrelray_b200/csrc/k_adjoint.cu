@@ -7,24 +7,31 @@
 // frozen at the forward run.  The forward steps run in the frame's precision
 // (TF = float: the FP32 PHYSICAL stepper with Kahan-compensated updates;
 // TF = double: FP64); the adjoint and the gradient reduction are FP64:
-//   1. forward: the PHYSICAL stepper runs the ray and saves its full state
-//      every ADJ_K accepted steps (checkpoints in HBM, per thread);
+//   1. forward: the PHYSICAL stepper runs the ray and stores, in HBM, the state
+//      and the step length of every accepted step (a window of `cap` steps per
+//      thread), and its full state at the start of each window (checkpoints);
 //   2. colour adjoint: dL/dc of the ray's sample through the SSAA combine,
 //      then lambda_N = dL/dc . dc/dy_N (+ the sphere-phase term) with c the
 //      bilinear sky or the sphere texture at the hit point;
-//   3. reverse: for each segment, last first, the steps are recomputed from
-//      the checkpoint (bit-identical: same stepper) in two levels - a pass
-//      that keeps a sub-checkpoint every ADJ_SUB steps, then, sub-segment by
-//      sub-segment, a pass that keeps the ADJ_SUB states - so a thread holds
-//      a few hundred bytes of states instead of a whole segment; lambda is
-//      pulled back through each step of x' = u, u' = G(x, u) in the stepper's
-//      form (only the velocity increments ku_i = h G(z_i) are kept: the
-//      stage points z_i are rebuilt from them, and their adjoints carry the
-//      position coupling); the products lambda^T dG/dz come from the
-//      geodesic's hand-written reverse sweep (geod_vjp.cuh);
+//   3. reverse: lambda is pulled back through each step, last first, from
+//      the stored states.  Rays longer than a window recompute the earlier ones
+//      from their checkpoints (bit-identical: same stepper).  Each step of
+//      x' = u, u' = G(x, u) is taken in the stepper's form (only the velocity
+//      increments ku_i = h G(z_i) are kept: the stage points z_i are rebuilt from
+//      them, and their adjoints carry the position coupling); the products
+//      lambda^T dG/dz come from the geodesic's hand-written reverse sweep
+//      (geod_vjp.cuh);
 //   4. lambda_0 is pulled back through the initial data (camera position,
 //      ray direction, null u^t), also by dual numbers.
 // Gradients are accumulated per thread and reduced in FP64.
+//
+// Bound: FP64 latency at 8 warps per SM (255 registers; 168 or 128 registers
+// measured 62 and 82 ms where this takes 59).  On 512x512 with FP32 steps the
+// sixth stage's zero products, two recompute passes per step and a fixed
+// assignment of rays to threads cost 117 ms; without them the kernel takes
+// 59 ms (256x256 with FP64 steps: 64.7 and 41.5 ms).  The states are 36 bytes
+// per FP32 step, 11 GB written and read per 512x512 gradient: 3.4 ms of HBM
+// time spread under the arithmetic.
 #include <cub/device/device_radix_sort.cuh>
 
 #include "dual.cuh"
@@ -114,7 +121,7 @@ __constant__ double c_beta[6] = {Fehlberg::b1, Fehlberg::b2, Fehlberg::b3, Fehlb
 // Stage point i of the Fehlberg step from y = (x, u), h and the velocity
 // increments ku_0..ku_{i-1} (x' = u is linear in the stages: phys_stepper.cuh):
 //   z_i^u = u + sum_m A_im ku_m,  z_i^x = x + h (c_i u + sum_m B_im ku_m).
-__device__ __forceinline__ void stage_point(const double y[8], double h, const double ku[6][4], int i, V4<double> &zx,
+__device__ __forceinline__ void stage_point(const double y[8], double h, const double ku[4][4], int i, V4<double> &zx,
                                             V4<double> &zu)
 {
     double sx[4], su[4];
@@ -136,9 +143,9 @@ __device__ __noinline__ void geod_vjp_call(const V4<double> &zx, const V4<double
 
 // lambda <- lambda . dPhi/dy at (y, h), Phi the 4th-order Fehlberg step
 //   u+ = u + sum_m K4_m ku_m,  x+ = x + h (u + sum_m beta_m ku_m);
-// th[0..1] += lambda . dPhi/d(spin, mass).  Only the six velocity increments
-// ku (24 doubles) and their adjoints (24 doubles) are kept; the stage points
-// are rebuilt from them.
+// th[0..1] += lambda . dPhi/d(spin, mass).  Only the first four velocity
+// increments ku (16 doubles) and the adjoints of the first five (20 doubles)
+// are kept; the stage points are rebuilt from them.
 __device__ void step_vjp(const Hot<double> &q, const double y[8], double h, double lam[8], double th[2])
 {
     if (q.metric == PRR_METRIC_FLAT) {  // G = 0: x+ = x + h u
@@ -146,25 +153,27 @@ __device__ void step_vjp(const Hot<double> &q, const double y[8], double h, doub
         for (int c = 0; c < 4; c++) lam[4 + c] += h * lam[c];
         return;
     }
-    double ku[6][4];
+    // The 4th-order step has no weight on the sixth stage (K46 = 0), so its adjoint is zero and the fifth
+    // increment, which only the sixth stage point uses, is not needed: four forward stages, five reverse ones.
+    double ku[4][4];
 #pragma unroll 1
-    for (int i = 0; i < 6; i++) {
+    for (int i = 0; i < 4; i++) {
         V4<double> zx, zu;
         stage_point(y, h, ku, i, zx, zu);
         const V4<double> g = geod_ks<double, true>(zx, zu, q.M, q.a);
         ku[i][0] = h * g.x; ku[i][1] = h * g.y; ku[i][2] = h * g.z; ku[i][3] = h * g.w;
     }
     // adjoints of the outputs: of ku_m, and of (x, u) through the direct terms
-    double kb[6][4], ox[4], ou[4];
+    double kb[5][4], ox[4], ou[4];
 #pragma unroll
     for (int c = 0; c < 4; c++) {
         ox[c] = lam[c];
         ou[c] = lam[4 + c] + h * lam[c];
 #pragma unroll
-        for (int m = 0; m < 6; m++) kb[m][c] = c_K4[m] * lam[4 + c] + h * c_beta[m] * lam[c];
+        for (int m = 0; m < 5; m++) kb[m][c] = c_K4[m] * lam[4 + c] + h * c_beta[m] * lam[c];
     }
 #pragma unroll 1
-    for (int i = 5; i >= 0; i--) {
+    for (int i = 4; i >= 0; i--) {
         V4<double> zx, zu;
         stage_point(y, h, ku, i, zx, zu);
         double gx[4], gu[4], gM, ga;
@@ -193,17 +202,17 @@ struct AdjointArgs {
     AdjParams ap;
     const float *dL_dimage;    // W*H*3 (device)
     const float *image;        // forward combined image W*H*3 (device)
-    void *ckpt;                // per thread: max_ckpt checkpoints (PhysRay<TF>)
+    void *ckpt;                // per thread: max_ckpt checkpoints (PhysRay<TF>), one per window
     int max_ckpt;
+    void *states;              // cap x ADJ_STATE values (TF) per thread, thread index fastest
+    int cap;                   // accepted steps per window
     double *grad;              // 5 doubles, accumulated
     unsigned long long *counters;
     long long nrays;
     const unsigned *order;     // ray visit order (null: 0, 1, 2, ...)
 };
 
-constexpr int ADJ_K = 64;    // accepted steps between checkpoints (HBM)
-constexpr int ADJ_SUB = 16;  // accepted steps between sub-checkpoints of the reverse sweep (per thread)
-static_assert(ADJ_K % ADJ_SUB == 0, "sub-segments tile a segment");
+constexpr int ADJ_STATE = 9;  // values stored per accepted step: the state before it (x, u) and its length h
 
 // At least PRR_ADJ_MINB resident CTAs of 128 threads per SM (caps registers).
 #ifndef PRR_ADJ_MINB
@@ -217,8 +226,8 @@ template <class TF> __device__ __forceinline__ void state8(const PhysRay<TF> &R,
 }
 
 // One RKF45 attempt of the adjoint's own forward steps.  The forward pass and
-// both recompute passes go through this one out-of-line copy, so a recomputed
-// segment repeats the forward steps bit for bit: inlined copies of the same
+// the recomputed windows go through this one out-of-line copy, so a recomputed
+// window repeats the forward steps bit for bit: inlined copies of the same
 // source may contract multiply-adds differently, and a recomputed step
 // sequence that drifts from the forward one would pull lambda back through
 // steps that were never taken.
@@ -229,9 +238,47 @@ __device__ __noinline__ int adj_attempt(const FrameParams &fp, const Hot<TF> &q,
     return phys_attempt<TF, 0>(fp, q, R, result, col, (TF)-1, &hit);
 }
 
+// lambda_N = gc . dc/dy_N of a ray that shows the sky (escaped) or sphere `hit`, and the direct phase term.
+template <class TF>
+__device__ __noinline__ void colour_adjoint(const FrameParams &fp, const AdjParams &ap, const PhysRay<TF> &R, bool escaped, int hit,
+                                            const double gc[3], double lam[8], double &phase_c)
+{
+    DC st[8];
+    double yN[8];
+    state8(R, yN);
+    for (int c = 0; c < 8; c++) st[c] = DC::var(yN[c], c);
+    V3<DC> cd;
+    if (escaped) {
+        cd = background_bilinear<DC>(fp.bg, st[4], st[5], st[6]);
+        if (!fp.bg.p || fp.bg_filter != PRR_BG_BILINEAR) cd = {DC(0.0), DC(0.0), DC(0.0)};  // RMS2X2 is piecewise constant
+    } else {
+        const DevSphere &Sp = fp.sph[hit];
+        DC cx = DC((double)Sp.cx), cy = DC((double)Sp.cy), cz = DC((double)Sp.cz);
+        if (hit == ap.sphere) {
+            DC ph = DC::var(ap.phase, 8 + P_PHASE);
+            cx = DC(ap.sph_R) * cos(ph); cy = DC(ap.sph_R) * sin(ph); cz = DC(ap.sph_z);
+        }
+        DC k = DC(1.0) / sqrt(st[4] * st[4] + st[5] * st[5] + st[6] * st[6]);
+        DC vx = st[4] * k, vy = st[5] * k, vz = st[6] * k;
+        DC v2 = vx * vx + vy * vy + vz * vz;
+        DC dx = st[0] - cx, dy = st[1] - cy, dz = st[2] - cz;
+        DC dvp = vx * dx + vy * dy + vz * dz;
+        DC disc = dvp * dvp - v2 * ((dx * dx + dy * dy + dz * dz) - DC((double)Sp.r * (double)Sp.r));
+        DC d = (DC(-2.0) * dvp - sqrt(disc)) / v2;
+        cd = sphere_colour_ad<DC>(Sp, cx, cy, cz, st[0], st[1], st[2], vx, vy, vz, d);
+    }
+    const DC *cc3 = &cd.x;
+    for (int c = 0; c < 3; c++) {
+        for (int j = 0; j < 8; j++) lam[j] += gc[c] * cc3[c].d[j];
+        phase_c += gc[c] * cc3[c].d[8 + P_PHASE];
+    }
+}
+
 template <class TF> __global__ void __launch_bounds__(128, PRR_ADJ_MINB) k_adjoint(AdjointArgs A)
 {
     const FrameParams &fp = *A.frame;
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
     const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long nth = (long long)gridDim.x * blockDim.x;
     PhysRay<TF> *ck = (PhysRay<TF> *)A.ckpt + tid * A.max_ckpt;
@@ -244,154 +291,148 @@ template <class TF> __global__ void __launch_bounds__(128, PRR_ADJ_MINB) k_adjoi
     double gacc[5] = {0, 0, 0, 0, 0};
     unsigned long long n_bad = 0, n_steps = 0;
     const int S = fp.samples;
-    TF ystore[ADJ_SUB][8], hstore[ADJ_SUB];
-    PhysRay<TF> sub[ADJ_K / ADJ_SUB];
-    for (long long k = tid; k < A.nrays; k += nth) {
-        const long long rid = A.order ? (long long)A.order[k] : k;
-        long long pix = rid / S;
-        int s = (int)(rid - pix * S);
-        int px = (int)(pix % fp.width), py = (int)(pix / fp.width);
-        // dL/dc through the SSAA combine (kernels/ssaa.cuh:116-130)
-        float uvx, uvy;
-        ray_uv(fp, px, py, s, uvx, uvy);
-        double y0[8], dy0[8][5];
-        initial_state(fp, A.ap, uvx, uvy, y0, dy0);
-        PhysRay<TF> R;
-        R.x = {(TF)y0[0], (TF)y0[1], (TF)y0[2], (TF)y0[3]};
-        R.u = {(TF)y0[4], (TF)y0[5], (TF)y0[6], (TF)y0[7]};
-        R.cx = {0, 0, 0, 0}; R.cu = {0, 0, 0, 0};
-        R.h = (TF)fp.h; R.trace_h = (TF)fp.h; R.l = 0; R.i = 0; R.accepted = 0; R.intersect = 0;
-        ck[0] = R;
-        int result = 0, hit = -1;
-        V3<float> col;
-        bool ok = true;
-        while (true) {
-            int before = R.accepted;
-            int st = adj_attempt<TF>(fp, qf, R, result, col, hit);
-            if (st == STEP_CONTINUE && R.accepted > before && R.accepted % ADJ_K == 0) {
-                int slot = R.accepted / ADJ_K;
-                if (slot >= A.max_ckpt) { ok = false; break; }
-                ck[slot] = R;
-            }
-            if (st != STEP_CONTINUE) break;
-        }
-        if (!ok) { n_bad++; continue; }
-        const int N = R.accepted;
-        n_steps += (unsigned long long)N;
-        bool escaped = result == PRR_RESULT_SUCCESS && metric_radius<TF>(fp, R.x.x, R.x.y, R.x.z) >= (TF)fp.rout;
-        if (!(escaped || result == PRR_RESULT_INTERSECTION)) continue;  // black: no gradient
-        // dL/dc for this sample
-        const float *gI = A.dL_dimage + 3 * pix;
-        const float *I = A.image + 3 * pix;
-        double gc[3];
-        const float cc[3] = {col.x, col.y, col.z};
-        bool any = false;
-        for (int c = 0; c < 3; c++) {
-            double d;
-            if (S == 1) d = (cc[c] > 0.0f && cc[c] < 1.0f) ? 1.0 : 0.0;
-            else d = (cc[c] * cc[c] > 0.0f && cc[c] * cc[c] < 1.0f && I[c] > 0.0f) ? (double)cc[c] / ((double)S * I[c]) : 0.0;
-            gc[c] = (double)gI[c] * d;
-            any |= gc[c] != 0.0;
-        }
-        if (!any) continue;
-        // lambda_N = gc . dc/dy_N ; direct phase term
+    // slot-major, thread index fastest: a warp's lanes, whose rays have similar lengths, read and write lines
+    TF *const mine = (TF *)A.states + tid;
+    auto slot = [&](int n, int c) -> TF & { return mine[((long long)(n % A.cap) * ADJ_STATE + c) * nth]; };
+    auto keep = [&](int n, const TF y[8], TF h) {
+#pragma unroll
+        for (int c = 0; c < 8; c++) slot(n, c) = y[c];
+        slot(n, 8) = h;
+    };
+    // A warp takes the next 32 rays of the order (longest first) when its last 32 are done.  Its lanes meet again after
+    // the forward steps and walk the reverse sweep by a common step index (idle where their ray is shorter): left to
+    // themselves they ran it in groups, at 21 of 32 lanes.
+    while (true) {
+        long long k = 0;
+        if (lane == 0) k = (long long)atomicAdd(&A.counters[C_WORK], 32ull);
+        k = __shfl_sync(FULL, k, 0);
+        if (k >= A.nrays) break;
+        k += lane;
+        int N = 0;  // steps to pull lambda back through; 0: no gradient (black, or no weight)
+        double dy0[8][5];
         double lam[8] = {0, 0, 0, 0, 0, 0, 0, 0}, th[2] = {0, 0}, phase_c = 0.0;
-        {
-            DC st[8];
-            double yN[8];
-            state8(R, yN);
-            for (int c = 0; c < 8; c++) st[c] = DC::var(yN[c], c);
-            V3<DC> cd;
-            if (escaped) {
-                cd = background_bilinear<DC>(fp.bg, st[4], st[5], st[6]);
-                if (!fp.bg.p || fp.bg_filter != PRR_BG_BILINEAR) cd = {DC(0.0), DC(0.0), DC(0.0)};  // RMS2X2 is piecewise constant
-            } else {
-                const DevSphere &Sp = fp.sph[hit];
-                DC cx = DC((double)Sp.cx), cy = DC((double)Sp.cy), cz = DC((double)Sp.cz);
-                if (hit == A.ap.sphere) {
-                    DC ph = DC::var(A.ap.phase, 8 + P_PHASE);
-                    cx = DC(A.ap.sph_R) * cos(ph); cy = DC(A.ap.sph_R) * sin(ph); cz = DC(A.ap.sph_z);
+        if (k < A.nrays) {
+            const long long rid = A.order ? (long long)A.order[k] : k;
+            long long pix = rid / S;
+            int s = (int)(rid - pix * S);
+            int px = (int)(pix % fp.width), py = (int)(pix / fp.width);
+            // dL/dc through the SSAA combine (kernels/ssaa.cuh:116-130)
+            float uvx, uvy;
+            ray_uv(fp, px, py, s, uvx, uvy);
+            double y0[8];
+            initial_state(fp, A.ap, uvx, uvy, y0, dy0);
+            PhysRay<TF> R;
+            R.x = {(TF)y0[0], (TF)y0[1], (TF)y0[2], (TF)y0[3]};
+            R.u = {(TF)y0[4], (TF)y0[5], (TF)y0[6], (TF)y0[7]};
+            R.cx = {0, 0, 0, 0}; R.cu = {0, 0, 0, 0};
+            R.h = (TF)fp.h; R.trace_h = (TF)fp.h; R.l = 0; R.i = 0; R.accepted = 0; R.intersect = 0;
+            ck[0] = R;
+            int result = 0, hit = -1;
+            V3<float> col;
+            bool ok = true;
+            while (true) {
+                const int before = R.accepted;
+                const TF yb[8] = {R.x.x, R.x.y, R.x.z, R.x.w, R.u.x, R.u.y, R.u.z, R.u.w};
+                const TF hb = R.h;
+                const int st = adj_attempt<TF>(fp, qf, R, result, col, hit);
+                if (R.accepted > before) {
+                    keep(before, yb, hb);
+                    if (st == STEP_CONTINUE && R.accepted % A.cap == 0) {
+                        const int w = R.accepted / A.cap;
+                        if (w >= A.max_ckpt) { ok = false; break; }
+                        ck[w] = R;
+                    }
                 }
-                DC k = DC(1.0) / sqrt(st[4] * st[4] + st[5] * st[5] + st[6] * st[6]);
-                DC vx = st[4] * k, vy = st[5] * k, vz = st[6] * k;
-                DC v2 = vx * vx + vy * vy + vz * vz;
-                DC dx = st[0] - cx, dy = st[1] - cy, dz = st[2] - cz;
-                DC dvp = vx * dx + vy * dy + vz * dz;
-                DC disc = dvp * dvp - v2 * ((dx * dx + dy * dy + dz * dz) - DC((double)Sp.r * (double)Sp.r));
-                DC d = (DC(-2.0) * dvp - sqrt(disc)) / v2;
-                cd = sphere_colour_ad<DC>(Sp, cx, cy, cz, st[0], st[1], st[2], vx, vy, vz, d);
-            }
-            const DC *cc3 = &cd.x;
-            for (int c = 0; c < 3; c++) {
-                for (int j = 0; j < 8; j++) lam[j] += gc[c] * cc3[c].d[j];
-                phase_c += gc[c] * cc3[c].d[8 + P_PHASE];
-            }
-        }
-        // reverse sweep, segment by segment, each in two recompute passes.  A
-        // recomputation that does not reach the steps the forward pass took
-        // (it cannot, as both run the same code, but it is checked rather than
-        // trusted) drops the ray: its states would be missing.
-        int r2 = 0, h2 = -1;
-        V3<float> c2;
-        bool consistent = true;
-        for (int seg = (N - 1) / ADJ_K; seg >= 0 && N > 0 && consistent; seg--) {
-            const int lo = seg * ADJ_K, hi = min(N, lo + ADJ_K);
-            const int nsub = (hi - lo + ADJ_SUB - 1) / ADJ_SUB;
-            // pass 1: the segment's sub-checkpoints
-            PhysRay<TF> Rs = ck[seg];
-            sub[0] = Rs;
-            while (Rs.accepted < lo + (nsub - 1) * ADJ_SUB) {
-                int st = adj_attempt<TF>(fp, qf, Rs, r2, c2, h2);
-                const int j = (Rs.accepted - lo) / ADJ_SUB;
-                if ((Rs.accepted - lo) % ADJ_SUB == 0 && j < nsub) sub[j] = Rs;
                 if (st != STEP_CONTINUE) break;
             }
-            if (Rs.accepted < lo + (nsub - 1) * ADJ_SUB) { consistent = false; break; }
-            // pass 2: each sub-segment, last first: keep its states, then pull lambda back
-            for (int j = nsub - 1; j >= 0; j--) {
-                Rs = sub[j];
-                const int slo = lo + j * ADJ_SUB, shi = min(hi, slo + ADJ_SUB);
-                while (Rs.accepted < shi) {
-                    const int before = Rs.accepted;
-                    TF yb[8] = {Rs.x.x, Rs.x.y, Rs.x.z, Rs.x.w, Rs.u.x, Rs.u.y, Rs.u.z, Rs.u.w};
-                    const TF hb = Rs.h;
-                    int st = adj_attempt<TF>(fp, qf, Rs, r2, c2, h2);
-                    if (Rs.accepted > before) {
-                        const int slot = before - slo;
-                        for (int c = 0; c < 8; c++) ystore[slot][c] = yb[c];
-                        hstore[slot] = hb;
-                    }
-                    if (st != STEP_CONTINUE) break;
+            if (ok) n_steps += (unsigned long long)R.accepted;
+            else n_bad++;
+            const bool escaped = result == PRR_RESULT_SUCCESS && metric_radius<TF>(fp, R.x.x, R.x.y, R.x.z) >= (TF)fp.rout;
+            if (ok && (escaped || result == PRR_RESULT_INTERSECTION)) {
+                // dL/dc for this sample
+                const float *gI = A.dL_dimage + 3 * pix;
+                const float *I = A.image + 3 * pix;
+                double gc[3];
+                const float cc[3] = {col.x, col.y, col.z};
+                bool any = false;
+                for (int c = 0; c < 3; c++) {
+                    double d;
+                    if (S == 1) d = (cc[c] > 0.0f && cc[c] < 1.0f) ? 1.0 : 0.0;
+                    else d = (cc[c] * cc[c] > 0.0f && cc[c] * cc[c] < 1.0f && I[c] > 0.0f) ? (double)cc[c] / ((double)S * I[c]) : 0.0;
+                    gc[c] = (double)gI[c] * d;
+                    any |= gc[c] != 0.0;
                 }
-                if (Rs.accepted != shi) { consistent = false; break; }
-                for (int n = shi - 1; n >= slo; n--) {
-                    double y[8];
-                    for (int c = 0; c < 8; c++) y[c] = (double)ystore[n - slo][c];
-                    step_vjp(q, y, (double)hstore[n - slo], lam, th);
+                if (any) {
+                    N = R.accepted;
+                    colour_adjoint<TF>(fp, A.ap, R, escaped, hit, gc, lam, phase_c);
                 }
             }
         }
-        if (!consistent) { n_bad++; continue; }
-        gacc[P_PHASE] += phase_c;
-        gacc[P_SPIN] += th[0];
-        gacc[P_MASS] += th[1];
-        for (int c = 0; c < 8; c++)
-            for (int p = 0; p < 5; p++) gacc[p] += lam[c] * dy0[c][p];
+        __syncwarp(FULL);
+        // reverse sweep, window by window; the last window's states are in
+        // place.  A recomputation that does not reach the steps the forward
+        // pass took (it cannot, as both run the same code, but it is checked
+        // rather than trusted) drops the ray: its states would be missing.
+        bool live = N > 0;
+        const int most = __reduce_max_sync(FULL, N);
+        for (int w = (most - 1) / A.cap; w >= 0 && most > 0; w--) {
+            const int lo = w * A.cap, hi = min(N, lo + A.cap);
+            if (live && N > lo + A.cap) {
+                int r2 = 0, h2 = -1;
+                V3<float> c2;
+                PhysRay<TF> Rs = ck[w];
+                while (Rs.accepted < hi) {
+                    const int before = Rs.accepted;
+                    const TF yb[8] = {Rs.x.x, Rs.x.y, Rs.x.z, Rs.x.w, Rs.u.x, Rs.u.y, Rs.u.z, Rs.u.w};
+                    const TF hb = Rs.h;
+                    const int st = adj_attempt<TF>(fp, qf, Rs, r2, c2, h2);
+                    if (Rs.accepted > before) keep(before, yb, hb);
+                    if (st != STEP_CONTINUE) break;
+                }
+                if (Rs.accepted != hi) live = false;
+            }
+            __syncwarp(FULL);
+            const int top = min(most, lo + A.cap) - 1, from = live ? hi : 0;  // this lane's steps: lo <= n < from
+            TF next[ADJ_STATE];
+            if (top < from) {
+#pragma unroll
+                for (int c = 0; c < ADJ_STATE; c++) next[c] = slot(top, c);
+            }
+#pragma unroll 1
+            for (int n = top; n >= lo; n--) {
+                double y[8];
+#pragma unroll
+                for (int c = 0; c < 8; c++) y[c] = (double)next[c];
+                const double h = (double)next[8];
+                if (n > lo && n - 1 < from) {  // the next state's loads fly during this step's products
+#pragma unroll
+                    for (int c = 0; c < ADJ_STATE; c++) next[c] = slot(n - 1, c);
+                }
+                if (n < from) step_vjp(q, y, h, lam, th);
+                __syncwarp(FULL);
+            }
+        }
+        if (N > 0 && !live) n_bad++;
+        if (live) {
+            gacc[P_PHASE] += phase_c;
+            gacc[P_SPIN] += th[0];
+            gacc[P_MASS] += th[1];
+            for (int c = 0; c < 8; c++)
+                for (int p = 0; p < 5; p++) gacc[p] += lam[c] * dy0[c][p];
+        }
     }
     for (int p = 0; p < 5; p++) {
         double v = gacc[p];
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
         if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(&A.grad[p], v);
     }
-    if (A.counters) {
-        if (n_bad) atomicAdd(&A.counters[C_MATH_ERROR], n_bad);
-        atomicAdd(&A.counters[C_ACCEPTED], n_steps);
-    }
+    if (n_bad) atomicAdd(&A.counters[C_MATH_ERROR], n_bad);
+    atomicAdd(&A.counters[C_ACCEPTED], n_steps);
 }
 
 cudaError_t launch_adjoint(const FrameParams *d_fp, const AdjointParamsHost &p, const float *dL, const float *image,
-                           void *ckpt, int max_ckpt, int threads_total, double *grad, unsigned long long *counters,
-                           long long nrays, const unsigned *order, int precision, cudaStream_t st)
+                           void *ckpt, int max_ckpt, void *states, int cap, int threads_total, double *grad,
+                           unsigned long long *counters, long long nrays, const unsigned *order, int precision, cudaStream_t st)
 {
     AdjointArgs A;
     A.frame = d_fp;
@@ -400,6 +441,8 @@ cudaError_t launch_adjoint(const FrameParams *d_fp, const AdjointParamsHost &p, 
     A.image = image;
     A.ckpt = ckpt;
     A.max_ckpt = max_ckpt;
+    A.states = states;
+    A.cap = cap;
     A.grad = grad;
     A.counters = counters;
     A.nrays = nrays;
@@ -446,6 +489,8 @@ size_t adjoint_checkpoint_bytes(int precision)
 {
     return precision == PRR_PREC_FP32 ? sizeof(PhysRay<float>) : sizeof(PhysRay<double>);
 }
+
+size_t adjoint_state_bytes(int precision) { return ADJ_STATE * (precision == PRR_PREC_FP32 ? sizeof(float) : sizeof(double)); }
 
 int adjoint_blocks_per_sm(int precision)
 {

@@ -108,8 +108,8 @@ struct AdjointParamsHost {
     int sphere;
 };
 cudaError_t launch_adjoint(const FrameParams *d_fp, const AdjointParamsHost &p, const float *dL, const float *image,
-                           void *ckpt, int max_ckpt, int threads_total, double *grad, unsigned long long *counters,
-                           long long nrays, const unsigned *order, int precision, cudaStream_t st);
+                           void *ckpt, int max_ckpt, void *states, int cap, int threads_total, double *grad,
+                           unsigned long long *counters, long long nrays, const unsigned *order, int precision, cudaStream_t st);
 // k_adjoint.cu: ray order for the adjoint, longest first: `order` receives the
 // ray indices sorted by descending accepted-step count `steps` (nrays
 // entries), so the rays a warp processes together have similar lengths.
@@ -117,8 +117,12 @@ cudaError_t launch_adjoint(const FrameParams *d_fp, const AdjointParamsHost &p, 
 size_t adjoint_order_bytes(long long nrays);
 cudaError_t launch_adjoint_order(const int *steps, long long nrays, unsigned *order, void *scratch, cudaStream_t st);
 size_t adjoint_checkpoint_bytes(int precision);
-int adjoint_blocks_per_sm(int precision);  // resident 128-thread CTAs of k_adjoint per SM
-constexpr int ADJ_CHECKPOINT_INTERVAL = 64;
+size_t adjoint_state_bytes(int precision);  // stored per thread and accepted step of a window
+int adjoint_blocks_per_sm(int precision);   // resident 128-thread CTAs of k_adjoint per SM
+// Accepted steps a thread stores (its window): longer rays recompute the earlier windows from checkpoints.  Most rays
+// of a frame take 1200 to 1400 steps (r + rout in steps of hmax), those that end on a sphere 1000 to 1500 more.
+constexpr int ADJ_WINDOW = 2048;
+constexpr int ADJ_WINDOW_MIN = 64;  // the window shrinks to this when device memory is short
 
 // fma_peak.cu
 cudaError_t launch_fma_peak(float *sink, int blocks, int threads, int iters, cudaStream_t st);

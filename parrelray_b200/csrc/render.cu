@@ -605,8 +605,16 @@ extern "C" prr_status prr_adjoint(prr_ctx *ctx, const prr_frame_desc *frame, con
         ap.phase = std::atan2((double)S.center[1], (double)S.center[0]);
         ap.sph_z = S.center[2];
     }
-    const int threads = ctx->nsm * adjoint_blocks_per_sm(prec) * 128;  // one resident wave
-    const int max_ckpt = d.max_steps / ADJ_CHECKPOINT_INTERVAL + 2;
+    // one resident wave, or fewer threads when there are fewer rays
+    const int threads = (int)std::min<long long>((long long)ctx->nsm * adjoint_blocks_per_sm(prec) * 128, (nrays + 127) / 128 * 128);
+    int cap = ADJ_WINDOW;
+    while (cap > ADJ_WINDOW_MIN && cap / 2 >= d.max_steps) cap /= 2;
+    while (ctx->adj_states.ensure((size_t)threads * cap * adjoint_state_bytes(prec)) != PRR_OK) {
+        cudaGetLastError();  // the failed allocation's, so the launches below do not report it
+        if (cap == ADJ_WINDOW_MIN) { ctx->err = "out of device memory for adjoint states"; return PRR_ERR_NOMEM; }
+        cap /= 2;
+    }
+    const int max_ckpt = d.max_steps / cap + 2;
     if ((s = alloc(ctx, ctx->adj_ckpt, (size_t)threads * max_ckpt * adjoint_checkpoint_bytes(prec), "adjoint checkpoints")) != PRR_OK) return s;
     if ((s = alloc(ctx, ctx->adj_dl, (size_t)npx * 3 * sizeof(float) + 8 * sizeof(double), "adjoint inputs")) != PRR_OK) return s;
     float *d_dl = (float *)ctx->adj_dl.p;
@@ -618,7 +626,7 @@ extern "C" prr_status prr_adjoint(prr_ctx *ctx, const prr_frame_desc *frame, con
     PRR_CK(ctx, cudaEventRecord(ctx->e0, st));
     PRR_CK(ctx, launch_adjoint_order(d_steps, nrays, d_order, d_sort_scratch, st));
     PRR_CK(ctx, launch_adjoint((const FrameParams *)ctx->frames.p, ap, d_dl, (const float *)ctx->image.p, ctx->adj_ckpt.p,
-                               max_ckpt, threads, d_grad, (unsigned long long *)ctx->counters.p, nrays, d_order, prec, st));
+                               max_ckpt, ctx->adj_states.p, cap, threads, d_grad, (unsigned long long *)ctx->counters.p, nrays, d_order, prec, st));
     PRR_CK(ctx, cudaEventRecord(ctx->e1, st));
     PRR_CK(ctx, cudaMemcpyAsync(grads, d_grad, 5 * sizeof(double), cudaMemcpyDeviceToHost, st));
     PRR_CK(ctx, cudaStreamSynchronize(st));
