@@ -37,6 +37,7 @@ struct prr_graph {
     int launches = 0;
     int bpsm = 1;
     prr_launch_config cfg{};
+    bool sample_items = false;  // the work items are rays (wants_sample_items)
     bool launched = false;
 };
 
@@ -82,7 +83,8 @@ prr_status record(prr_graph *g, cudaStream_t st)
     a.frames = (const FrameParams *)g->frames.p;
     a.frame_pix_begin = (const long long *)g->frame_begin.p;
     a.nframes = n;
-    a.total_pixels = plan.total_pixels;
+    a.total_pixels = g->sample_items ? plan.total_rays : plan.total_pixels;
+    a.sample_items = g->sample_items;
     a.counters = (unsigned long long *)g->counters.p;
     a.geod_table = ctx->geod_table == 1;
     a.hamiltonian = ctx->hamiltonian;
@@ -110,14 +112,20 @@ prr_status record(prr_graph *g, cudaStream_t st)
         return PRR_OK;
     }
     a.rgb8 = g->d_rgb8;
+    if (g->sample_items) a.sample_rgb = (float *)g->sample_rgb.p;
     PRR_GCK(g, launch_persistent(a, plan.precision, g->cfg.block_size, g->bpsm, ctx->nsm, st));
     g->launches += 1;
     for (int f = 0; f < n; f++) {
         const FrameParams &p = plan.fp[f];
         const size_t npx = (size_t)p.width * p.height;
         float *img = image + 3 * p.pix_begin;
-        if (p.fxaa) {
-            PRR_GCK(g, launch_finish(img, p.width, p.height, 1, g->d_rgbf ? g->d_rgbf + 3 * p.pix_begin : nullptr,
+        const bool combine = g->sample_items && p.samples > 1;
+        if (combine) {
+            PRR_GCK(g, launch_combine(a.sample_rgb + 3 * p.ray_begin, p.width, p.height, p.samples, img, st));
+            g->launches += 1;
+        }
+        if (p.fxaa || combine) {
+            PRR_GCK(g, launch_finish(img, p.width, p.height, p.fxaa, g->d_rgbf ? g->d_rgbf + 3 * p.pix_begin : nullptr,
                                      g->d_rgb8 ? g->d_rgb8 + 3 * p.pix_begin : nullptr, st));
             g->launches += 1;
         } else if (g->d_rgbf) {
@@ -132,7 +140,7 @@ prr_status upload(prr_graph *g)
     const RenderPlan &plan = g->plan;
     const size_t n = plan.fp.size();
     PRR_GCK(g, cudaMemcpy(g->frames.p, plan.fp.data(), n * sizeof(FrameParams), cudaMemcpyHostToDevice));
-    PRR_GCK(g, cudaMemcpy(g->frame_begin.p, plan.pix_begin.data(), (n + 1) * sizeof(long long), cudaMemcpyHostToDevice));
+    PRR_GCK(g, cudaMemcpy(g->frame_begin.p, (g->sample_items ? plan.ray_begin : plan.pix_begin).data(), (n + 1) * sizeof(long long), cudaMemcpyHostToDevice));
     return PRR_OK;
 }
 
@@ -169,6 +177,11 @@ extern "C" prr_status prr_graph_create(prr_ctx *ctx, const prr_frame_desc *frame
         (s = galloc(g, g->counters, C_COUNT * sizeof(unsigned long long), "counters")) != PRR_OK ||
         (s = galloc(g, g->image, (size_t)plan.total_pixels * 3 * sizeof(float), "image")) != PRR_OK) {
         release(g); delete g; return s;
+    }
+    g->sample_items = wants_sample_items(ctx, plan, g->cfg);
+    if (g->sample_items && g->sample_rgb.ensure((size_t)plan.total_rays * 3 * sizeof(float)) != PRR_OK) {
+        cudaGetLastError();  // short of device memory: pixels as work items (SPLIT fails just below)
+        g->sample_items = false;
     }
     if (plan.precision == PRR_PREC_SPLIT &&
         ((s = galloc(g, g->sample_rgb, (size_t)plan.total_rays * 3 * sizeof(float), "per-sample colours")) != PRR_OK ||

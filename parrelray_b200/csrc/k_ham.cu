@@ -578,6 +578,7 @@ __device__ __forceinline__ bool ham_flag(const PersistentArgs &a, HSlot<float> &
     if ((long long)slot < a.fp64_capacity) a.fp64_queue[slot] = ((unsigned long long)sl.frame << 40) | (unsigned long long)rid;
     float *o = a.sample_rgb + 3 * (fp.ray_begin + rid);
     o[0] = o[1] = o[2] = 0.f;
+    if (a.sample_items) return true;
     sl.s += 1;
     if (sl.s < sl.S) {
         ham_init<float, true>(fp, sl, sl.s);
@@ -623,6 +624,7 @@ __device__ __forceinline__ bool ham_finish(const PersistentArgs &a, HSlot<T> &sl
         const long long rid = ((long long)sl.py * fp.width + sl.px) * sl.S + sl.s;
         float *o = a.sample_rgb + 3 * (fp.ray_begin + rid);
         o[0] = col.x; o[1] = col.y; o[2] = col.z;
+        if (a.sample_items) return true;
         sl.s += 1;
         if (sl.s < sl.S) {
             ham_init<T, true>(fp, sl, sl.s);
@@ -630,6 +632,7 @@ __device__ __forceinline__ bool ham_finish(const PersistentArgs &a, HSlot<T> &sl
         }
         return true;
     }
+    if (a.sample_items && sl.S > 1) return true;
     if (sl.S == 1) {
         sl.acc0 = fminf(fmaxf(col.x, 0.f), 1.f); sl.acc1 = fminf(fmaxf(col.y, 0.f), 1.f); sl.acc2 = fminf(fmaxf(col.z, 0.f), 1.f);
     } else {
@@ -655,15 +658,20 @@ __device__ __forceinline__ void ham_start(const PersistentArgs &a, HSlot<T> &sl,
 {
     sl.frame = find_frame_h(a.frame_pix_begin, a.nframes, it);
     const FrameParams &fp = a.frames[sl.frame];
-    const long long p = it - __ldg(a.frame_pix_begin + sl.frame);
-    sl.px = (int)(p % fp.width);
-    sl.py = (int)(p / fp.width);
+    long long p = it - __ldg(a.frame_pix_begin + sl.frame);
     sl.S = fp.samples;
     sl.s = 0;
+    if (a.sample_items && sl.S > 1) { sl.s = (int)(p % sl.S); p /= sl.S; }
+    // bands of 4 rows, each walked in tiles of 8 pixels: a warp's lanes start as neighbours in both directions, so more of
+    // them are quick together (FP64 960x540 26.1 -> 24.8 ms, disk 640x640 12.3 -> 12.0 ms; a row of 32 before)
+    const int band = (int)(p / (4ll * fp.width)), j = (int)(p - 4ll * fp.width * band), rows = min(4, fp.height - 4 * band);
+    const int tile = j / (8 * rows), k = j - 8 * rows * tile, cols = min(8, fp.width - 8 * tile);
+    sl.px = 8 * tile + k % cols;
+    sl.py = 4 * band + k / cols;
     sl.acc0 = sl.acc1 = sl.acc2 = 0.f;
     sl.q = make_hot<T>(fp);
     sl.flag_r = SPLIT ? (float)(fp.fp64_rfac * kerr_r_plus<T>(sl.q.M, sl.q.a)) : -1.0f;
-    ham_init<T, SPLIT, EMIS>(fp, sl, 0);
+    ham_init<T, SPLIT, EMIS>(fp, sl, sl.s);
     sl.busy = true;
 }
 

@@ -284,6 +284,13 @@ cudaError_t launch_persistent(const PersistentArgs &a, int precision, int block,
     return launch_pair(a, a.rays_per_thread == 2 ? 2 : 1, false, block, blocks_per_sm, nsm, st);
 }
 
+bool renders_with_ham(int precision, int geod_table, int hamiltonian, int rays_per_thread, int emission)
+{
+    if (precision == PRR_PREC_FP64) return (hamiltonian & PRR_HAM_FP64) != 0;
+    if (!(hamiltonian & PRR_HAM_FP32)) return false;
+    return precision == PRR_PREC_SPLIT || (!geod_table && (rays_per_thread != 2 || emission));
+}
+
 int persistent_occupancy(int precision, int geod_table, int block, int rays_per_thread, int emission, int hamiltonian)
 {
     int n = 0;

@@ -41,9 +41,9 @@ cudaError_t launch_finish(const float *image, int w, int h, int fxaa, float *out
 // k_persistent.cu: PHYSICAL-mode persistent renderer over a batch of frames.
 struct PersistentArgs {
     const FrameParams *frames;   // device array
-    const long long *frame_pix_begin;  // device array, nframes+1 prefix of pixel counts
+    const long long *frame_pix_begin;  // device array, nframes+1 prefix of the frames' work items: pixels, or rays (sample_items)
     int nframes;
-    long long total_pixels;      // work items (pixels over all frames)
+    long long total_pixels;      // work items over all frames
     float *image;                // combined FP32 image, 3 floats/pixel (all frames)
     uint8_t *rgb8;               // optional direct quantised output (frames without FXAA)
     float *sample_rgb;           // per-sample colours (split precision; optional otherwise)
@@ -58,6 +58,8 @@ struct PersistentArgs {
     int rays_per_thread;         // FP32: pixel slots in flight per thread (1 or 2; 0 = 1)
     int *ray_steps;              // optional: accepted steps per ray (not k_pair; single frame)
     int emission;                // 1 = some frame has plasma emission (the kernels with emission.cuh)
+    int sample_items;            // k_ham: 1 = a work item is a ray, not a pixel: colours of frames with several samples go
+                                 // to sample_rgb (launch_combine follows)
     int hamiltonian;             // PRR_HAM_FP32 | PRR_HAM_FP64 mask: renders that integrate (x, p) in Hamiltonian form (k_ham.cu)
 };
 // Dispatches to the kernel of the precision: FP32 with one pixel slot per
@@ -67,6 +69,9 @@ struct PersistentArgs {
 // rays_per_thread slots per thread); other FP64 renders and the
 // Christoffel-table variant -> k_persistent.
 cudaError_t launch_persistent(const PersistentArgs &a, int precision, int block, int blocks_per_sm, int nsm, cudaStream_t st);
+
+// k_persistent.cu: whether launch_persistent picks k_ham.
+bool renders_with_ham(int precision, int geod_table, int hamiltonian, int rays_per_thread, int emission);
 
 // k_persistent.cu: resident CTAs per SM of the kernel launch_persistent picks.
 int persistent_occupancy(int precision, int geod_table, int block, int rays_per_thread = 1, int emission = 0,

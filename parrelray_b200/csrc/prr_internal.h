@@ -81,6 +81,7 @@ struct RenderPlan {
     int mode = PRR_MODE_PHYSICAL;
     int precision = PRR_PREC_FP32;
     bool any_fxaa = false;
+    bool any_ssaa = false;      // some frame has several samples per pixel
     bool any_emission = false;  // some frame has plasma emission
     bool plugin = false;        // the frames use metric plug-ins (then every frame does)
 };
@@ -100,6 +101,8 @@ prr_status run_plan(prr_ctx *ctx, const RenderPlan &plan, uint8_t *d_rgb8, float
 // Single frame: per-ray states and per-sample colours to host buffers.
 prr_status trace_plan(prr_ctx *ctx, const RenderPlan &plan, float *h_state, double *h_state64, float *h_rgb);
 prr_status collect_stats(prr_ctx *ctx, const RenderPlan &plan, prr_stats *stats);
+// Do the work items of a persistent launch of this plan under `cfg` be rays (k_ham's sample_items) rather than pixels?
+bool wants_sample_items(const prr_ctx *ctx, const RenderPlan &plan, const prr_launch_config &cfg);
 // Resident CTAs per SM of the persistent kernel under the context's launch
 // configuration (its blocks_per_sm, or the occupancy limit when that is 0).
 int resolve_bpsm(prr_ctx *ctx, int precision, bool emission = false);

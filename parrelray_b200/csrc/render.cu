@@ -135,6 +135,7 @@ prr_status build_plan(prr_ctx *ctx, const prr_frame_desc *frames, int n, RenderP
     plan.mode = frames[0].mode;
     plan.precision = frames[0].precision;
     plan.any_fxaa = false;
+    plan.any_ssaa = false;
     plan.any_emission = false;
     plan.plugin = false;
     for (int f = 0; f < n; f++) {
@@ -258,6 +259,7 @@ prr_status build_plan(prr_ctx *ctx, const prr_frame_desc *frames, int n, RenderP
         plan.pix_begin[f + 1] = plan.pix_begin[f] + npx;
         plan.ray_begin[f + 1] = plan.ray_begin[f] + npx * d.samples;
         if (d.fxaa) plan.any_fxaa = true;
+        if (d.samples > 1) plan.any_ssaa = true;
     }
     plan.total_pixels = plan.pix_begin[n];
     plan.total_rays = plan.ray_begin[n];
@@ -265,7 +267,19 @@ prr_status build_plan(prr_ctx *ctx, const prr_frame_desc *frames, int n, RenderP
     return PRR_OK;
 }
 
-static prr_status upload_plan(prr_ctx *ctx, const RenderPlan &plan, cudaStream_t st)
+// A ray is the finer work item: a pixel's samples run in series on one lane, so with few pixels per lane, or with
+// samples of very different lengths (a ray that grazes a sphere takes up to 10000 attempts), lanes idle behind them.
+// It costs the 12 bytes per ray of the per-sample colours and the combine pass that reads them: 1920x1080x4 Kerr frame
+// 180 -> 170 ms, 640x360x9 57 -> 42 ms.  Up to 2^28 rays a call (3.2 GB of colours), beyond which no lane runs out of
+// pixels early.  Emission frames keep pixels: the compiler starts a pixel's later samples with other contractions
+// than its first in that instantiation, and prr_render_noalloc (pixels) gives the same bytes as prr_render.
+bool wants_sample_items(const prr_ctx *ctx, const RenderPlan &plan, const prr_launch_config &cfg)
+{
+    return plan.any_ssaa && !plan.any_emission && plan.total_rays <= (1LL << 28) &&
+           renders_with_ham(plan.precision, ctx->geod_table == 1, ctx->hamiltonian, cfg.rays_per_thread, plan.any_emission);
+}
+
+static prr_status upload_plan(prr_ctx *ctx, const RenderPlan &plan, cudaStream_t st, bool sample_items = false)
 {
     size_t n = plan.fp.size();
     prr_status s;
@@ -273,21 +287,22 @@ static prr_status upload_plan(prr_ctx *ctx, const RenderPlan &plan, cudaStream_t
     if ((s = alloc(ctx, ctx->frame_begin, (n + 1) * sizeof(long long), "frame table")) != PRR_OK) return s;
     if ((s = alloc(ctx, ctx->counters, C_COUNT * sizeof(unsigned long long), "counters")) != PRR_OK) return s;
     PRR_CK(ctx, cudaMemcpyAsync(ctx->frames.p, plan.fp.data(), n * sizeof(FrameParams), cudaMemcpyHostToDevice, st));
-    PRR_CK(ctx, cudaMemcpyAsync(ctx->frame_begin.p, plan.pix_begin.data(), (n + 1) * sizeof(long long), cudaMemcpyHostToDevice, st));
+    PRR_CK(ctx, cudaMemcpyAsync(ctx->frame_begin.p, (sample_items ? plan.ray_begin : plan.pix_begin).data(), (n + 1) * sizeof(long long), cudaMemcpyHostToDevice, st));
     PRR_CK(ctx, cudaMemsetAsync(ctx->counters.p, 0, C_COUNT * sizeof(unsigned long long), st));
     // the host vectors may be freed when the caller returns: make the copies complete first
     PRR_CK(ctx, cudaStreamSynchronize(st));
     return PRR_OK;
 }
 
-static PersistentArgs persistent_args(prr_ctx *ctx, const RenderPlan &plan)
+static PersistentArgs persistent_args(prr_ctx *ctx, const RenderPlan &plan, bool sample_items)
 {
     PersistentArgs a;
     memset(&a, 0, sizeof(a));
     a.frames = (const FrameParams *)ctx->frames.p;
     a.frame_pix_begin = (const long long *)ctx->frame_begin.p;
     a.nframes = (int)plan.fp.size();
-    a.total_pixels = plan.total_pixels;
+    a.total_pixels = sample_items ? plan.total_rays : plan.total_pixels;
+    a.sample_items = sample_items;
     a.counters = (unsigned long long *)ctx->counters.p;
     a.geod_table = ctx->geod_table == 1;
     a.hamiltonian = ctx->hamiltonian;
@@ -314,7 +329,13 @@ prr_status run_plan(prr_ctx *ctx, const RenderPlan &plan, uint8_t *d_rgb8, float
 {
     prr_status s = check_emission_schedule(ctx, plan);
     if (s != PRR_OK) return s;
-    s = upload_plan(ctx, plan, st);
+    const bool persistent = plan.mode != PRR_MODE_REFERENCE && ctx->schedule != PRR_SCHED_PLAIN && !plan.plugin;
+    bool sample_items = persistent && wants_sample_items(ctx, plan, ctx->cfg);
+    if (sample_items && plan.precision != PRR_PREC_SPLIT && ctx->sample_rgb.ensure((size_t)plan.total_rays * 3 * sizeof(float)) != PRR_OK) {
+        cudaGetLastError();  // short of device memory: pixels as work items need no per-sample colours
+        sample_items = false;
+    }
+    s = upload_plan(ctx, plan, st, sample_items);
     if (s != PRR_OK) return s;
     const int n = (int)plan.fp.size();
     unsigned long long *counters = (unsigned long long *)ctx->counters.p;
@@ -339,7 +360,7 @@ prr_status run_plan(prr_ctx *ctx, const RenderPlan &plan, uint8_t *d_rgb8, float
     };
 
     bool trace_timed = false;
-    if (plan.mode == PRR_MODE_REFERENCE || ctx->schedule == PRR_SCHED_PLAIN || plan.plugin) {
+    if (!persistent) {
         long long max_rays = 0;
         for (const auto &p : plan.fp) max_rays = std::max(max_rays, (long long)p.width * p.height * p.samples);
         if ((s = alloc(ctx, ctx->sample_rgb, (size_t)max_rays * 3 * sizeof(float), "per-sample colours")) != PRR_OK) return s;
@@ -367,7 +388,7 @@ prr_status run_plan(prr_ctx *ctx, const RenderPlan &plan, uint8_t *d_rgb8, float
         }
     } else {
         trace_timed = timed;
-        PersistentArgs a = persistent_args(ctx, plan);
+        PersistentArgs a = persistent_args(ctx, plan, sample_items);
         a.image = image;
         const int bpsm = resolve_bpsm(ctx, plan.precision, plan.any_emission);
         if (plan.precision == PRR_PREC_SPLIT) {
@@ -389,12 +410,20 @@ prr_status run_plan(prr_ctx *ctx, const RenderPlan &plan, uint8_t *d_rgb8, float
             }
         } else {
             a.rgb8 = d_rgb8;
+            if (sample_items) a.sample_rgb = (float *)ctx->sample_rgb.p;
             if (timed) PRR_CK(ctx, cudaEventRecord(ctx->t0, st));
             PRR_CK(ctx, launch_persistent(a, plan.precision, ctx->cfg.block_size, bpsm, ctx->nsm, st));
             if (timed) PRR_CK(ctx, cudaEventRecord(ctx->t1, st));
             launches++;
-            for (int f = 0; f < n; f++)
-                if ((s = finish(f, true)) != PRR_OK) return s;
+            for (int f = 0; f < n; f++) {
+                const FrameParams &p = plan.fp[f];
+                const bool combine = sample_items && p.samples > 1;
+                if (combine) {
+                    PRR_CK(ctx, launch_combine(a.sample_rgb + 3 * p.ray_begin, p.width, p.height, p.samples, image + 3 * p.pix_begin, st));
+                    launches++;
+                }
+                if ((s = finish(f, !combine)) != PRR_OK) return s;
+            }
         }
     }
     if (timed) {
@@ -419,7 +448,11 @@ prr_status trace_plan(prr_ctx *ctx, const RenderPlan &plan, float *h_state, doub
     cudaStream_t st = ctx->stream;
     prr_status s = check_emission_schedule(ctx, plan);
     if (s != PRR_OK) return s;
-    s = upload_plan(ctx, plan, st);
+    const int prec = plan.precision == PRR_PREC_FP64 ? PRR_PREC_FP64 : PRR_PREC_FP32;
+    const bool sample_items = plan.mode != PRR_MODE_REFERENCE && !plan.plugin && !(ctx->schedule == PRR_SCHED_PLAIN && !h_state64) &&
+                              plan.any_ssaa && !plan.any_emission &&
+                              renders_with_ham(prec, ctx->geod_table == 1, ctx->hamiltonian, ctx->cfg.rays_per_thread, plan.any_emission);
+    s = upload_plan(ctx, plan, st, sample_items);
     if (s != PRR_OK) return s;
     const FrameParams &p = plan.fp[0];
     const long long nr = (long long)p.width * p.height * p.samples;
@@ -447,12 +480,11 @@ prr_status trace_plan(prr_ctx *ctx, const RenderPlan &plan, float *h_state, doub
         ctx->last_launches = launches;
     } else {
         if ((s = alloc(ctx, ctx->image, (size_t)plan.total_pixels * 3 * sizeof(float), "image")) != PRR_OK) return s;
-        PersistentArgs a = persistent_args(ctx, plan);
+        PersistentArgs a = persistent_args(ctx, plan, sample_items);
         a.image = (float *)ctx->image.p;
         a.sample_rgb = rgb;
         if (h_state64) a.ray_state64 = (double *)ctx->state.p;
         else a.ray_state = (float *)ctx->state.p;
-        int prec = plan.precision == PRR_PREC_FP64 ? PRR_PREC_FP64 : PRR_PREC_FP32;
         PRR_CK(ctx, launch_persistent(a, prec, ctx->cfg.block_size, resolve_bpsm(ctx, prec, plan.any_emission), ctx->nsm, st));
         ctx->last_launches = 1;
     }
