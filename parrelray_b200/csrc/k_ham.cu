@@ -131,6 +131,41 @@ PRR_DEV void ham_rhs(P2<T> P, P2<T> Q, P2<T> W, const HamConst<T> &c, P2<T> &dP,
     dW = f2(fma_(neg_(fL), lz, pz), mul_(fL, fma_(Lam, dgzh, dLz)));
 }
 
+// h dy/dlambda in FP64, where every operation is a DP slot (the kernel keeps the FP64 pipe busy 81 % of the cycles) and
+// nothing has to round as FP32 did: with S = r^2 + a^2 z^2/r^2 and Sigma = r^4 + a^2 z^2 = r^2 S, one reciprocal (1/q)
+// serves beside the two square roots, t = r^3/Sigma = r/S, f = 2M t, grad r = (x, y, z q/r^2) t, l and the gradient of
+// l.p share r/q and a/q, and h enters once: 77 operations where the form above takes 92 (and 6 more for two Newton
+// steps in place of one third-order step per root).  640x360 frame in FP64 14.5 -> 11.9 ms with 6 CTAs per SM.
+PRR_DEV void ham_rhs_h(double2 P, double2 Q, double2 W, const HamConst<double> &c, double h, double2 &kP, double2 &kQ, double2 &kW)
+{
+    const double X = P.x, Y = P.y, z = W.x, px = Q.x, py = Q.y, pz = W.y;
+    const double Z2 = z * z;
+    const double hb = fma_(0.5, fma_(X, X, fma_(Y, Y, Z2)), c.nha2);  // (R^2 - a^2)/2
+    const double S2h = fma_(hb, hb, c.a2 * Z2);                       // (S/2)^2
+    const double iSh = h3_rsqrt(S2h);                                   // 2/S
+    const double r2 = fma_(S2h, iSh, hb);
+    const double ir = h3_rsqrt(r2), r = r2 * ir;
+    const double q = r2 + c.a2, iq = h3_rcp(q);
+    const double iS = 0.5 * iSh, irS = iS * ir, t = iS * r, f = c.M2 * t;
+    const double riq = r * iq, aiq = c.a * iq;
+    const double drx = X * t, dry = Y * t, drz = (z * q) * irS;
+    // grad f / (2 f) = (3/(2r) - 2 r^3/Sigma) grad r - (0, 0, a^2 z/Sigma), 1/Sigma = irS / r
+    const double cc = fma_(-2.0, t, 1.5 * ir);
+    const double lz = z * ir;
+    const double dgx = cc * drx, dgy = cc * dry, dgz = fma_(cc, drz, -((c.a2 * lz) * irS));
+    const double lx = fma_(riq, X, aiq * Y), ly = fma_(riq, Y, -(aiq * X));
+    const double lp = fma_(px, lx, py * ly);
+    const double Lam = fma_(lz, pz, lp) - c.pt;
+    // gradient of l.p at fixed p: grad r times ((x p_x + y p_y) - 2 r lp)/q - p_z z/r^2, plus the explicit part
+    const double Pp = fma_(fma_(px, X, py * Y), iq, -fma_(2.0, riq * lp, (lz * ir) * pz));
+    const double dLx = fma_(drx, Pp, fma_(riq, px, -(aiq * py))), dLy = fma_(dry, Pp, fma_(riq, py, aiq * px));
+    const double dLz = fma_(drz, Pp, pz * ir);
+    const double hfL = h * (f * Lam);
+    kP = f2(fma_(-hfL, lx, h * px), fma_(-hfL, ly, h * py));
+    kQ = f2(hfL * fma_(Lam, dgx, dLx), hfL * fma_(Lam, dgy, dLy));
+    kW = f2(fma_(-hfL, lz, h * pz), hfL * fma_(Lam, dgz, dLz));
+}
+
 // u = dx/dlambda (spatial) and u^t = -p_t + f Lam at (x, p), with IEEE
 // square roots: used by the sphere test, the sky lookup and the outputs.
 template <class T> PRR_DEV V4<T> ham_velocity(T x, T y, T z, T px, T py, T pz, const HamConst<T> &c)
@@ -275,9 +310,13 @@ template <class T> PRR_DEV HamStep<T> ham_stages(const HamRay<T> &R, const HamCo
 #define PC(v) sp((T)(v))
 #define RHS(kP, kQ, kW, zP, zQ, zW)                                                                                    \
     {                                                                                                                  \
-        V dP_, dQ_, dW_;                                                                                               \
-        ham_rhs<T>(zP, zQ, zW, c, dP_, dQ_, dW_);                                                                      \
-        kP = mul_(H, dP_); kQ = mul_(H, dQ_); kW = mul_(H, dW_);                                                        \
+        if constexpr (sizeof(T) == 8) {                                                                                \
+            ham_rhs_h(zP, zQ, zW, c, h, kP, kQ, kW);                                                                   \
+        } else {                                                                                                       \
+            V dP_, dQ_, dW_;                                                                                           \
+            ham_rhs<T>(zP, zQ, zW, c, dP_, dQ_, dW_);                                                                  \
+            kP = mul_(H, dP_); kQ = mul_(H, dQ_); kW = mul_(H, dW_);                                                    \
+        }                                                                                                              \
     }
     V k1P, k1Q, k1W, k2P, k2Q, k2W, k3P, k3Q, k3W, k4P, k4Q, k4W, k5P, k5Q, k5W, k6P, k6Q, k6W;
     RHS(k1P, k1Q, k1W, P, Q, W)
@@ -678,15 +717,16 @@ __device__ __forceinline__ void ham_start(const PersistentArgs &a, HSlot<T> &sl,
 }  // namespace
 
 // Resident CTAs per SM the small-CTA (<= 64 threads) instantiations are
-// built for: FP32 8 (128 registers, no spills); FP64 8 as well (128
-// registers, 458 bytes of spills that stay in L1): the FP64 form is latency
-// bound, and on the 1080p frame 8 CTAs measured 871 ms, 6 (168 registers)
-// 922 ms, 4 (192 registers, no spills) 1100 ms.
+// built for: FP32 8 (128 registers, no spills), at the FMA pipe's limit (76 %
+// of its cycles) from 4 CTAs on: 960x540x4 frame 42.6 ms with 8, 44.5 with 6,
+// 43.7 with 4; FP64 6 (168 registers), which a small frame's long rays like
+// better than 8 (128 registers and spills): 960x540 frame 21.0 ms against
+// 23.7, uneven batch 36.4 against 36.4, 5 CTAs 21.5 and 36.3.
 #ifndef PRR_HAM_SMALL_MINB
 #define PRR_HAM_SMALL_MINB 8
 #endif
 #ifndef PRR_HAM_SMALL_MINB_F64
-#define PRR_HAM_SMALL_MINB_F64 8
+#define PRR_HAM_SMALL_MINB_F64 6
 #endif
 template <class T> constexpr int ham_small_minb() { return sizeof(T) == 8 ? PRR_HAM_SMALL_MINB_F64 : PRR_HAM_SMALL_MINB; }
 
