@@ -134,9 +134,13 @@ prr_status prr_create(int device, prr_ctx **out)
         delete ctx;
         return PRR_ERR_CUDA;
     }
-    ctx->cfg.block_size = 128;
+    // The launch shape of a context that was not tuned: the one prr_autotune settles on for full-size frames.  Against
+    // 128-thread CTAs refilled after every attempt (what it was): 1920x1080x4 Kerr frame 257 -> 170 ms, FP64 960x540
+    // 33 -> 21 ms, split batch 114 -> 70 ms, 640x360x9 56 -> 43 ms, disk 640x640 14.5 -> 12.0 ms; a 320x180 frame, which
+    // does not fill the chip, 2.4 -> 2.5 ms.
+    ctx->cfg.block_size = 64;
     ctx->cfg.blocks_per_sm = 0;  // 0: occupancy-derived
-    ctx->cfg.compaction_interval = 1;
+    ctx->cfg.compaction_interval = 64;
     ctx->cfg.rays_per_thread = 1;
     ctx->schedule = PRR_SCHED_PERSISTENT;
     *out = ctx;
