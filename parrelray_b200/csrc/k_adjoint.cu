@@ -25,13 +25,13 @@
 //      ray direction, null u^t), also by dual numbers.
 // Gradients are accumulated per thread and reduced in FP64.
 //
-// Bound: FP64 latency at 8 warps per SM (255 registers; 168 or 128 registers
-// measured 62 and 82 ms where this takes 59).  On 512x512 with FP32 steps the
-// sixth stage's zero products, two recompute passes per step and a fixed
-// assignment of rays to threads cost 117 ms; without them the kernel takes
-// 59 ms (256x256 with FP64 steps: 64.7 and 41.5 ms).  The states are 36 bytes
-// per FP32 step, 11 GB written and read per 512x512 gradient: 3.4 ms of HBM
-// time spread under the arithmetic.
+// Bound: FP64 latency at 8 (FP64 steps) or 12 warps per SM.  On 512x512 with
+// FP32 steps the sixth stage's zero products, two recompute passes per step
+// and a fixed assignment of rays to threads cost 117 ms, without them 59 ms,
+// and with the closed forms of geod_vjp.cuh 37 ms (256x256 with FP64 steps:
+// 64.7, 41.5 and 31.4 ms).  The states are 36 bytes per FP32 step, 11 GB
+// written and read per 512x512 gradient: 3.4 ms of HBM time spread under the
+// arithmetic.
 #include <cub/device/device_radix_sort.cuh>
 
 #include "dual.cuh"
@@ -134,13 +134,6 @@ __device__ __forceinline__ void stage_point(const double y[8], double h, const d
     zu = {su[0], su[1], su[2], su[3]};
 }
 
-// The geodesic's reverse sweep, one copy in the kernel (called at every stage).
-__device__ __noinline__ void geod_vjp_call(const V4<double> &zx, const V4<double> &zu, double M, double a,
-                                           const double w[4], double gx[4], double gu[4], double &gM, double &ga)
-{
-    geod_vjp(zx, zu, M, a, w, gx, gu, gM, ga);
-}
-
 // lambda <- lambda . dPhi/dy at (y, h), Phi the 4th-order Fehlberg step
 //   u+ = u + sum_m K4_m ku_m,  x+ = x + h (u + sum_m beta_m ku_m);
 // th[0..1] += lambda . dPhi/d(spin, mass).  Only the first four velocity
@@ -155,43 +148,54 @@ __device__ void step_vjp(const Hot<double> &q, const double y[8], double h, doub
     }
     // The 4th-order step has no weight on the sixth stage (K46 = 0), so its adjoint is zero and the fifth
     // increment, which only the sixth stage point uses, is not needed: four forward stages, five reverse ones.
+    const double hm = 2.0 * q.M * h;  // geod_unit and geod_vjp leave the 2M to the step length
     double ku[4][4];
-#pragma unroll 1
+#pragma unroll
     for (int i = 0; i < 4; i++) {
         V4<double> zx, zu;
         stage_point(y, h, ku, i, zx, zu);
-        const V4<double> g = geod_ks<double, true>(zx, zu, q.M, q.a);
-        ku[i][0] = h * g.x; ku[i][1] = h * g.y; ku[i][2] = h * g.z; ku[i][3] = h * g.w;
+        const V4<double> g = geod_unit(zx, zu, q.M, q.a);
+        ku[i][0] = hm * g.x; ku[i][1] = hm * g.y; ku[i][2] = hm * g.z; ku[i][3] = hm * g.w;
     }
     // adjoints of the outputs: of ku_m, and of (x, u) through the direct terms
     double kb[5][4], ox[4], ou[4];
 #pragma unroll
     for (int c = 0; c < 4; c++) {
-        ox[c] = lam[c];
-        ou[c] = lam[4 + c] + h * lam[c];
+        // (lam[3], of the coordinate time, is zero throughout: no colour and no acceleration depends on it)
+        ox[c] = c < 3 ? lam[c] : 0.0;
+        ou[c] = lam[4 + c] + h * ox[c];
 #pragma unroll
-        for (int m = 0; m < 5; m++) kb[m][c] = c_K4[m] * lam[4 + c] + h * c_beta[m] * lam[c];
+        for (int m = 0; m < 5; m++) kb[m][c] = c_K4[m] * lam[4 + c] + (h * c_beta[m]) * ox[c];
     }
 #pragma unroll 1
     for (int i = 4; i >= 0; i--) {
         V4<double> zx, zu;
         stage_point(y, h, ku, i, zx, zu);
-        double gx[4], gu[4], gM, ga;
+        double gx[3], gu[4], gM, ga;
         const double wv[4] = {kb[i][0], kb[i][1], kb[i][2], kb[i][3]};
-        geod_vjp_call(zx, zu, q.M, q.a, wv, gx, gu, gM, ga);
-        th[0] += h * ga;
+        geod_vjp(zx, zu, q.M, q.a, wv, gx, gu, gM, ga);
+        th[0] += hm * ga;
         th[1] += h * gM;
-        double zbx[4], zbu[4];
+        // adjoints of the stage point (nothing depends on the coordinate time)
+        double zbx[3], zbu[4];
 #pragma unroll
         for (int c = 0; c < 4; c++) {
-            zbx[c] = h * gx[c];
-            zbu[c] = h * gu[c];
-            ox[c] += zbx[c];
-            ou[c] += zbu[c] + h * c_c[i] * zbx[c];
+            zbu[c] = hm * gu[c];
+            ou[c] += zbu[c];
         }
-        for (int m = 0; m < i; m++)
 #pragma unroll
-            for (int c = 0; c < 4; c++) kb[m][c] += c_A[i][m] * zbu[c] + h * c_B[i][m] * zbx[c];
+        for (int c = 0; c < 3; c++) {
+            zbx[c] = hm * gx[c];
+            ox[c] += zbx[c];
+            ou[c] += h * c_c[i] * zbx[c];
+        }
+        for (int m = 0; m < i; m++) {
+            const double A = c_A[i][m], hB = h * c_B[i][m];
+#pragma unroll
+            for (int c = 0; c < 4; c++) kb[m][c] += A * zbu[c];
+#pragma unroll
+            for (int c = 0; c < 3; c++) kb[m][c] += hB * zbx[c];
+        }
     }
 #pragma unroll
     for (int c = 0; c < 4; c++) { lam[c] = ox[c]; lam[4 + c] = ou[c]; }
@@ -214,10 +218,11 @@ struct AdjointArgs {
 
 constexpr int ADJ_STATE = 9;  // values stored per accepted step: the state before it (x, u) and its length h
 
-// At least PRR_ADJ_MINB resident CTAs of 128 threads per SM (caps registers).
-#ifndef PRR_ADJ_MINB
-#define PRR_ADJ_MINB 1
-#endif
+// Resident CTAs of 128 threads per SM the kernel is built for (caps the
+// registers): FP32 steps 3 (168 registers: 36.8 ms on 512x512 against 38.9
+// with 255), FP64 steps 2 (255 registers: 31.4 ms on 256x256 against 38.8
+// with 168).
+template <class TF> constexpr int adj_minb() { return sizeof(TF) == 4 ? 3 : 2; }
 
 template <class TF> __device__ __forceinline__ void state8(const PhysRay<TF> &R, double y[8])
 {
@@ -274,7 +279,7 @@ __device__ __noinline__ void colour_adjoint(const FrameParams &fp, const AdjPara
     }
 }
 
-template <class TF> __global__ void __launch_bounds__(128, PRR_ADJ_MINB) k_adjoint(AdjointArgs A)
+template <class TF> __global__ void __launch_bounds__(128, adj_minb<TF>()) k_adjoint(AdjointArgs A)
 {
     const FrameParams &fp = *A.frame;
     constexpr unsigned FULL = 0xffffffffu;
