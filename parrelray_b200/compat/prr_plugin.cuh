@@ -118,6 +118,7 @@ struct PluginHooks {
 #else
     static constexpr bool kSpherical = false;
 #endif
+    static constexpr bool kErrorBound = false;  // a header's geodesic has no known error bound
     Camera cam;
     Spacetime space;
     Tracer trace;

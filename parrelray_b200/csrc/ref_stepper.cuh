@@ -87,9 +87,37 @@ PRR_DEV void ref_metric(const FrameParams &fp, const RefRay &R, float g[16])
     else metric_ks<float>(R.r.x, R.r.y, R.r.z, fp.metric == PRR_METRIC_FLAT ? 0.0f : fp.M, fp.a, g);
 }
 
+// Can Sphere::intersects pass on some sphere for a ray at p, with a window up to hmax?  (far2 bounds |p - c|^2 of a
+// hit, render.cu:build_plan; it covers hmax only, so a larger first step always tests.)
+PRR_DEV bool ref_near(const FrameParams &fp, const V4<float> &p)
+{
+    bool near = fp.h > fp.hmax;
+    for (int s = 0; s < fp.nspheres; s++) {
+        const float dx = p.x - fp.sph[s].cx, dy = p.y - fp.sph[s].cy, dz = p.z - fp.sph[s].cz;
+        near |= !(dx * dx + dy * dy + dz * dz > fp.sph[s].far2);
+    }
+    return near;
+}
+
+// Is the error of a step h from (x, u) under half of eps whatever the sixth stage says?  With U the largest component
+// of u, s = h U / r <= 1/16, h <= 1/4 and r >= 4M, the embedded difference of this mode's stages (whose velocity
+// inputs use h u where h du belongs) is at most h U (0.01 h + 0.2 s M / r), twice its maximum over 6e6 random states
+// of all signs, masses and spins; the two seven-term FP32 sums it is taken from add up to 12 half ulps of the largest
+// coordinate (time included).  Then 0.9 h (eps/err)^0.2 > h, so a step of hmax is accepted and followed by hmax.
+PRR_DEV bool ref_small_error(const FrameParams &fp, const V4<float> &x, const V4<float> &u, float h)
+{
+    const float U = fmaxf(fmaxf(fabsf(u.x), fabsf(u.y)), fmaxf(fabsf(u.z), fabsf(u.w)));
+    const float a = fp.metric == PRR_METRIC_KERR ? fp.a : 0.0f, M = fp.metric == PRR_METRIC_FLAT ? 0.0f : fp.M;
+    const float R2 = x.x * x.x + x.y * x.y + x.z * x.z, r2 = 0.999f * (R2 - a * a);  // under the Kerr-Schild r^2
+    const float ir = sfu_rsqrt(r2), hU = h * U, s = hU * ir;
+    const float X = sfu_rsqrt(R2) * R2 + fabsf(x.w) + U;
+    return r2 >= 16.1f * M * M && s <= 0.0625f && h <= 0.25f && hU * (0.01f * h + 0.2f * s * M * ir) + 7.2e-7f * X <= 0.5f * fp.eps;
+}
+
 // User_UPDATE
 PRR_DEV bool ref_update(const FrameParams &fp, RefRay &R, float h)
 {
+    if (!ref_near(fp, R.r)) return true;
     Hit c = intersect_scene<float>(fp, R.r.x, R.r.y, R.r.z, R.u.x, R.u.y, R.u.z, h);
     if (c.hit) { R.result = PRR_RESULT_INTERSECTION; return false; }
     return true;
@@ -100,6 +128,7 @@ PRR_DEV bool ref_endloop(const FrameParams &fp, RefRay &R, float th)
 {
     float r = metric_radius<float>(fp, R.r.x, R.r.y, R.r.z);
     if (r >= fp.rout || (fp.metric != PRR_METRIC_FLAT && r <= fp.rstop)) { R.result = PRR_RESULT_SUCCESS; return false; }
+    if (!ref_near(fp, R.r)) return true;
     Hit c = intersect_scene<float>(fp, R.r.x, R.r.y, R.r.z, R.u.x, R.u.y, R.u.z, th);
     if (c.hit) { R.u = {c.r, c.g, c.b, 0.0f}; R.result = PRR_RESULT_INTERSECTION; return false; }
     return true;
@@ -107,6 +136,8 @@ PRR_DEV bool ref_endloop(const FrameParams &fp, RefRay &R, float th)
 
 struct BuiltinHooks {
     static constexpr bool kSpherical = false;  // Cartesian (x, y, z, t) states
+    static constexpr bool kErrorBound = true;  // small_error holds for the metric (ref_small_error)
+    PRR_DEV bool small_error(const V4<float> &x, const V4<float> &u, float h) const { return ref_small_error(fp, x, u, h); }
     const FrameParams &fp;
     PRR_DEV void metric(const RefRay &R, float g[16]) const { ref_metric(fp, R, g); }
     PRR_DEV V4<float> geod(const V4<float> &x, const V4<float> &u) const { return ref_geod(fp, x, u); }
@@ -123,6 +154,8 @@ template <class H> PRR_DEV void ref_rkf_h(const FrameParams &fp, const H &hk, Re
     float h = fp.h, hmin = fp.hmin, hmax = fp.hmax, _h = h, eps = fp.eps, trace_h = fp.h;
     V4<float> x = R.r, u = R.u, _x = x, _u = u, __x, __u;
     bool intersect = false;
+    // eps so tight that the stages' own error or the sums' rounding leave no room: do not look (ref_small_error)
+    const bool bounded = 0.002f * hmax * hmax + 4e-5f <= 0.5f * eps;
     int i = 0;
     for (float l = 0.0f; l < 1000.0f;) {
         i += 1;
@@ -140,20 +173,29 @@ template <class H> PRR_DEV void ref_rkf_h(const FrameParams &fp, const H &hk, Re
         V4<float> z5x = v4add(v4add(v4add(v4add(x, v4scl(K::A51, kx1)), v4scl(K::A52, kx2)), v4scl(K::A53, kx3)), v4scl(K::A54, kx4));
         V4<float> z5u = v4add(v4add(v4add(v4add(u, v4scl(K::A51, kx1)), v4scl(K::A52, ku2)), v4scl(K::A53, ku3)), v4scl(K::A54, ku4));
         V4<float> kx5 = v4scl(h, z5u), ku5 = v4scl(h, hk.geod(z5x, z5u));
-        V4<float> z6x = v4add(v4add(v4add(v4add(v4add(x, v4scl(K::A61, kx1)), v4scl(K::A62, kx2)), v4scl(K::A63, kx3)), v4scl(K::A64, kx4)), v4scl(K::A65, kx5));
-        V4<float> z6u = v4add(v4add(v4add(v4add(v4add(u, v4scl(K::A61, kx1)), v4scl(K::A62, ku2)), v4scl(K::A63, ku3)), v4scl(K::A64, ku4)), v4scl(K::A65, ku5));
-        V4<float> kx6 = v4scl(h, z6u), ku6 = v4scl(h, hk.geod(z6x, z6u));
+        _x = v4add(v4add(v4add(v4add(v4add(x, v4scl(K::K41, kx1)), v4scl(K::K42, kx2)), v4scl(K::K43, kx3)), v4scl(K::K44, kx4)), v4scl(K::K45, kx5));
+        _u = v4add(v4add(v4add(v4add(v4add(u, v4scl(K::K41, ku1)), v4scl(K::K42, ku2)), v4scl(K::K43, ku3)), v4scl(K::K44, ku4)), v4scl(K::K45, ku5));
+        // The sixth stage (zero weight in _x, _u) and the error decide nothing in intersection mode, nor where they are
+        // known to leave an hmax step at hmax; a warp evaluates them when one of its lanes needs them.
+        bool quiet = intersect && i <= 10000;
+        if constexpr (H::kErrorBound) quiet = quiet || (bounded && h == hmax && hk.small_error(x, u, h));
+        float maxerr = 0.0f;
+        _h = hmax;
+        if (__any_sync(__activemask(), !quiet)) {
+            V4<float> z6x = v4add(v4add(v4add(v4add(v4add(x, v4scl(K::A61, kx1)), v4scl(K::A62, kx2)), v4scl(K::A63, kx3)), v4scl(K::A64, kx4)), v4scl(K::A65, kx5));
+            V4<float> z6u = v4add(v4add(v4add(v4add(v4add(u, v4scl(K::A61, kx1)), v4scl(K::A62, ku2)), v4scl(K::A63, ku3)), v4scl(K::A64, ku4)), v4scl(K::A65, ku5));
+            V4<float> kx6 = v4scl(h, z6u), ku6 = v4scl(h, hk.geod(z6x, z6u));
+            _x = v4add(_x, v4scl(K::K46, kx6));
+            _u = v4add(_u, v4scl(K::K46, ku6));
+            __x = v4add(v4add(v4add(v4add(v4add(v4add(x, v4scl(K::K51, kx1)), v4scl(K::K52, kx2)), v4scl(K::K53, kx3)), v4scl(K::K54, kx4)), v4scl(K::K55, kx5)), v4scl(K::K56, kx6));
+            __u = v4add(v4add(v4add(v4add(v4add(v4add(u, v4scl(K::K51, ku1)), v4scl(K::K52, ku2)), v4scl(K::K53, ku3)), v4scl(K::K54, ku4)), v4scl(K::K55, ku5)), v4scl(K::K56, ku6));
 
-        _x = v4add(v4add(v4add(v4add(v4add(v4add(x, v4scl(K::K41, kx1)), v4scl(K::K42, kx2)), v4scl(K::K43, kx3)), v4scl(K::K44, kx4)), v4scl(K::K45, kx5)), v4scl(K::K46, kx6));
-        _u = v4add(v4add(v4add(v4add(v4add(v4add(u, v4scl(K::K41, ku1)), v4scl(K::K42, ku2)), v4scl(K::K43, ku3)), v4scl(K::K44, ku4)), v4scl(K::K45, ku5)), v4scl(K::K46, ku6));
-        __x = v4add(v4add(v4add(v4add(v4add(v4add(x, v4scl(K::K51, kx1)), v4scl(K::K52, kx2)), v4scl(K::K53, kx3)), v4scl(K::K54, kx4)), v4scl(K::K55, kx5)), v4scl(K::K56, kx6));
-        __u = v4add(v4add(v4add(v4add(v4add(v4add(u, v4scl(K::K51, ku1)), v4scl(K::K52, ku2)), v4scl(K::K53, ku3)), v4scl(K::K54, ku4)), v4scl(K::K55, ku5)), v4scl(K::K56, ku6));
-
-        float ex = fmaxf(fmaxf(fmaxf(fabsf(__x.x - _x.x), fabsf(__x.y - _x.y)), fabsf(__x.z - _x.z)), fabsf(__x.w - _x.w));
-        float eu = fmaxf(fmaxf(fmaxf(fabsf(__u.x - _u.x), fabsf(__u.y - _u.y)), fabsf(__u.z - _u.z)), fabsf(__u.w - _u.w));
-        float maxerr = fmaxf(ex, eu);
-        _h = 0.9f * h * powf(eps / maxerr, 0.2f);
-        _h = fminf(fmaxf(_h, hmin), hmax);
+            float ex = fmaxf(fmaxf(fmaxf(fabsf(__x.x - _x.x), fabsf(__x.y - _x.y)), fabsf(__x.z - _x.z)), fabsf(__x.w - _x.w));
+            float eu = fmaxf(fmaxf(fmaxf(fabsf(__u.x - _u.x), fabsf(__u.y - _u.y)), fabsf(__u.z - _u.z)), fabsf(__u.w - _u.w));
+            maxerr = fmaxf(ex, eu);
+            _h = 0.9f * h * powf(eps / maxerr, 0.2f);
+            _h = fminf(fmaxf(_h, hmin), hmax);
+        }
 
         if (intersect && i > 10000) intersect = false;
         if (i > 1000000) break;
