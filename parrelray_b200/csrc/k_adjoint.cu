@@ -29,7 +29,7 @@
 // FP32 steps the sixth stage's zero products, two recompute passes per step
 // and a fixed assignment of rays to threads cost 117 ms, without them 59 ms,
 // and with the closed forms of geod_vjp.cuh 37 ms (256x256 with FP64 steps:
-// 64.7, 41.5 and 31.4 ms).  The states are 36 bytes per FP32 step, 11 GB
+// 64.7, 41.5, 31.5 and, with adj_attempt's rule, 27.4 ms).  The states are 36 bytes per FP32 step, 11 GB
 // written and read per 512x512 gradient: 3.4 ms of HBM time spread under the
 // arithmetic.
 #include <cub/device/device_radix_sort.cuh>
@@ -236,11 +236,38 @@ template <class TF> __device__ __forceinline__ void state8(const PhysRay<TF> &R,
 // source may contract multiply-adds differently, and a recomputed step
 // sequence that drifts from the forward one would pull lambda back through
 // steps that were never taken.
+// FP64 steps evaluate the sixth stage and the error only where they can
+// decide something (cruise_radius, r2 its square for R^2; nor in intersection
+// mode, which accepts hmin steps whatever the error until its 10000 attempts
+// are used up), for a warp when one of its lanes needs them: 256x256 gradient
+// 31.5 -> 27.4 ms.  FP32 steps run beside the FP64 sweeps of other warps and
+// gain nothing from it (512x512: 36.9 against 37.4 ms, with more spills).
 template <class TF>
-__device__ __noinline__ int adj_attempt(const FrameParams &fp, const Hot<TF> &q, PhysRay<TF> &R, int &result,
+__device__ __noinline__ int adj_attempt(const FrameParams &fp, const Hot<TF> &q, PhysRay<TF> &R, float r2, int &result,
                                         V3<float> &col, int &hit)
 {
-    return phys_attempt<TF, 0>(fp, q, R, result, col, (TF)-1, &hit);
+    bool full = true;
+    if constexpr (sizeof(TF) == 8) {
+        const bool quiet = (R.intersect && R.i < 10000) ||
+                           (R.h == q.hmax && (float)(R.x.x * R.x.x + R.x.y * R.x.y + R.x.z * R.x.z) >= r2);
+        full = __any_sync(__activemask(), !quiet);
+    }
+    return phys_attempt<TF, 0>(fp, q, R, result, col, (TF)-1, &hit, nullptr, full);
+}
+
+// cruise_radius^2 + a^2 (bounds the Kerr-Schild r by the Euclidean R) for the initial state y, infinite when y is not null.
+__device__ float adj_cruise_r2(const FrameParams &fp, double M, double a, const double y[8], float noise)
+{
+    double g[16], p[4], n = 0.0, t = 0.0;
+    metric_ks<double>(y[0], y[1], y[2], M, a, g);
+    for (int m = 0; m < 4; m++) {
+        p[m] = g[4 * m] * y[4] + g[4 * m + 1] * y[5] + g[4 * m + 2] * y[6] + g[4 * m + 3] * y[7];
+        n += p[m] * y[4 + m];
+        t += fabs(p[m] * y[4 + m]);
+    }
+    if (!(fabs(n) <= 1e-3 * t)) return INFINITY;
+    const float r = cruise_radius(fp, fabsf((float)p[3]), (float)M, noise);
+    return 1.0001f * (r * r + (float)(a * a));
 }
 
 // lambda_N = gc . dc/dy_N of a ray that shows the sky (escaped) or sphere `hit`, and the direct phase term.
@@ -316,6 +343,7 @@ template <class TF> __global__ void __launch_bounds__(128, adj_minb<TF>()) k_adj
         int N = 0;  // steps to pull lambda back through; 0: no gradient (black, or no weight)
         double dy0[8][5];
         double lam[8] = {0, 0, 0, 0, 0, 0, 0, 0}, th[2] = {0, 0}, phase_c = 0.0;
+        float cr2 = INFINITY;
         if (k < A.nrays) {
             const long long rid = A.order ? (long long)A.order[k] : k;
             long long pix = rid / S;
@@ -331,6 +359,7 @@ template <class TF> __global__ void __launch_bounds__(128, adj_minb<TF>()) k_adj
             R.u = {(TF)y0[4], (TF)y0[5], (TF)y0[6], (TF)y0[7]};
             R.cx = {0, 0, 0, 0}; R.cu = {0, 0, 0, 0};
             R.h = (TF)fp.h; R.trace_h = (TF)fp.h; R.l = 0; R.i = 0; R.accepted = 0; R.intersect = 0;
+            if constexpr (sizeof(TF) == 8) cr2 = adj_cruise_r2(fp, q.M, q.a, y0, cruise_noise<TF>());
             ck[0] = R;
             int result = 0, hit = -1;
             V3<float> col;
@@ -339,7 +368,7 @@ template <class TF> __global__ void __launch_bounds__(128, adj_minb<TF>()) k_adj
                 const int before = R.accepted;
                 const TF yb[8] = {R.x.x, R.x.y, R.x.z, R.x.w, R.u.x, R.u.y, R.u.z, R.u.w};
                 const TF hb = R.h;
-                const int st = adj_attempt<TF>(fp, qf, R, result, col, hit);
+                const int st = adj_attempt<TF>(fp, qf, R, cr2, result, col, hit);
                 if (R.accepted > before) {
                     keep(before, yb, hb);
                     if (st == STEP_CONTINUE && R.accepted % A.cap == 0) {
@@ -390,7 +419,7 @@ template <class TF> __global__ void __launch_bounds__(128, adj_minb<TF>()) k_adj
                     const int before = Rs.accepted;
                     const TF yb[8] = {Rs.x.x, Rs.x.y, Rs.x.z, Rs.x.w, Rs.u.x, Rs.u.y, Rs.u.z, Rs.u.w};
                     const TF hb = Rs.h;
-                    const int st = adj_attempt<TF>(fp, qf, Rs, r2, c2, h2);
+                    const int st = adj_attempt<TF>(fp, qf, Rs, cr2, r2, c2, h2);
                     if (Rs.accepted > before) keep(before, yb, hb);
                     if (st != STEP_CONTINUE) break;
                 }

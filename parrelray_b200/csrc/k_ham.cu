@@ -204,30 +204,19 @@ template <class T> struct HSlot {
     EmisRay<T> E;  // emission kernels only
 };
 
-// Where a step of hmax needs no error estimate.  The propagated 4th-order solution has no weight on the sixth
-// stage (K46 = 0): that stage, the embedded difference, the scaled norm and the step control are about a quarter of
-// an attempt and only decide accept/reject and the next step.  With r the Kerr-Schild radius and hE = h |p_t|, over
-// all null (x, p) with r >= 4M, |a| <= M and s = hE / r <= 1/8 the embedded difference of one step is at most
-//     0.8 M s^5 in x and 1.4 (M / r) |p_t| s^5 in p
-// (maximum over 10^7 random states in FP64; it falls with r and with s).  The radius returned keeps five times
-// those bounds under atol / 4 and requires the FP32 rounding of the difference, at most 2.5e-7 hE (seven half-ulp
-// roundings per stage increment, sum |E_i| = 0.118), to be under 0.3 atol: then err < 0.9^5 (atol alone is a lower
-// bound of every scale), so the attempt is accepted and 0.9 hmax err^(-1/5) is clamped to hmax, exactly what the
-// full evaluation decides.  Infinite where that cannot be shown (atol = 0, very tight tolerances, initial data that
-// are not null).  The test on the Euclidean radius, R^2 >= radius^2 + a^2, implies r >= radius.
+// Squared Euclidean radius from which a step of hmax needs no error estimate (cruise_radius; R^2 >= radius^2 + a^2
+// implies r >= radius).  The propagated 4th-order solution has no weight on the sixth stage (K46 = 0): that stage, the
+// embedded difference, the scaled norm and the step control are about a quarter of an attempt and only decide
+// accept/reject and the next step.  Infinite for initial data that are not null.
 // The kernel is issue bound (FP64: also by the power and the six reciprocals of the norm), so the work left out is
 // time: 1920x1080x4 Kerr frame 257.0 -> 217.3 ms, 640x360 in FP64 24.7 -> 15.9 ms, split batch 46.4 -> 38.8 ms, the
 // same bits out.  A warp evaluates the error when one of its lanes needs it (lanes near the hole, mostly).
 template <class T> __device__ __forceinline__ T ham_cruise_r2(const FrameParams &fp, T M, T a, const T u[4], const T p[4])
 {
-    const float E = fabsf((float)p[3]), hE = mul_(fp.hmax, E), atol = fp.atol;
-    const float noise = sizeof(T) == 4 ? 2.5e-7f : 5e-16f;
     const float n0 = (float)mul_(p[0], u[0]), n1 = (float)mul_(p[1], u[1]), n2 = (float)mul_(p[2], u[2]), n3 = (float)mul_(p[3], u[3]);
     const bool null = fabsf(n0 + n1 + n2 + n3) <= 1e-3f * (fabsf(n0) + fabsf(n1) + fabsf(n2) + fabsf(n3));
-    if (!(null && atol > 0.0f && noise * hE <= 0.3f * atol)) return T(INFINITY);
-    const float m = (float)M, h5 = hE * hE * hE * hE * hE / (0.25f * atol);
-    const float rx = __powf(4.0f * m * h5, 0.2f), rp = __powf(7.0f * m * E * h5, 1.0f / 6.0f);
-    const float r = 1.001f * fmaxf(fmaxf(4.0f * m, 8.0f * hE), fmaxf(rx, rp));
+    const float r = cruise_radius(fp, fabsf((float)p[3]), (float)M, cruise_noise<T>());
+    if (!null) return T(INFINITY);
     return fma_(a, a, (T)mul_(r, r));  // (explicit: a shared a * a would change how the compiler contracts ham_init)
 }
 

@@ -154,3 +154,32 @@ def test_fp64_rays_take_the_steps_of_a_full_estimator(gpu, kw):
         s, pt, h, path, acc, j = s[:, k], pt[k], h[k], path[k], acc[k], j[k]
     same = count == state[:, 11]
     assert same.mean() >= 0.98, (same.mean(), stats.as_dict())
+
+
+@pytest.mark.parametrize("tol,hmax,M", [(1e-6, 0.1, 1.0), (1e-8, 0.05, 0.2), (1e-5, 0.5, 2.0)])
+def test_velocity_form_stays_under_the_step_control_too(tol, hmax, M):
+    """The (x, u) form of the adjoint's FP64 steps (phys_stepper.cuh, cruise_radius) under the same radius."""
+    from test_reference_error_skip import accel
+
+    rng = np.random.default_rng(13)
+    n = 40_000
+    a = M * rng.uniform(0.0, 1.0, n) * rng.choice([-1.0, 1.0], n)
+    d = rng.normal(size=(3, n))
+    d /= np.sqrt((d * d).sum(0))
+    lo = float(rule_radius(M, 1.0, hmax, tol, 5e-16))
+    r = lo * np.exp(rng.uniform(0.0, 3.5, n) * (np.arange(n) % 2))
+    ct, ph = rng.uniform(-1, 1, n), rng.uniform(0, 2 * np.pi, n)
+    st, R = np.sqrt(1 - ct * ct), np.sqrt(r * r + a * a)
+    x = np.stack((R * st * np.cos(ph), R * st * np.sin(ph), r * ct))
+    _, f, l = ks(*x, M, a)
+    ld = (np.stack(l) * d).sum(0)
+    rt = np.sqrt(4 * f * f * ld * ld - 4 * (f - 1) * (1 + f * ld * ld))
+    ut = np.maximum((-2 * f * ld + rt) / (2 * (f - 1)), (-2 * f * ld - rt) / (2 * (f - 1)))
+    u = np.concatenate((d, ut[None])) / (ut - f * (ld + ut))  # E = 1
+    y = np.concatenate((x, np.zeros((1, n)), u))
+    k = []
+    for row in A:
+        z = y + sum((c * kk for c, kk in zip(row, k)), 0 * y)
+        k.append(hmax * np.concatenate((z[4:], accel(z[:4], z[4:], M, a))))
+    e = sum((c5 - c4) * kk for c5, c4, kk in zip(B5, B4, k))
+    assert (np.abs(e) / tol).max() < 0.9**5
