@@ -140,11 +140,15 @@ PRR_DEV void emis_step(const FrameParams &fp, T M, T a, const V4<T> &x, const V4
 // Hamiltonian form of the FP32 renderer): k.u_e = p_mu u_e^mu needs no
 // lowering, so nu_e = -u_e^t (p_i v^i + p_t); p_t is the constant of the
 // motion.  Same model, same arithmetic otherwise.
+// R2 = x^2 + y^2 + z^2: as R^2 - a^2 <= r^2 <= R^2, it tells most points
+// outside the shell without the two square roots of r (disk 640x640 frame,
+// camera at r = 50, shell to r = 20: 11.95 -> 11.65 ms).
 template <class T>
-PRR_DEV void emis_step_p(const FrameParams &fp, T M, T a, T x, T y, T z, T px, T py, T pz, T pt, T h, EmisRay<T> &E)
+PRR_DEV void emis_step_p(const FrameParams &fp, T M, T a, T x, T y, T z, T px, T py, T pz, T pt, T h, T R2, EmisRay<T> &E)
 {
     const EmisParams &e = fp.em;
     if (e.kind == PRR_EMISSION_NONE) return;
+    if ((float)R2 > 1.0001f * __fmaf_rn((float)a, (float)a, __fmul_rn(e.r_out, e.r_out))) return;
     const T r = ks_radius<T>(x, y, z, a);
     if (!(r >= (T)e.r_in && r <= (T)e.r_out)) return;  // outside the emitting shell: f and l are not needed
     T f, l[3];

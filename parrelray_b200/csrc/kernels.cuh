@@ -58,6 +58,7 @@ struct PersistentArgs {
     int rays_per_thread;         // FP32: pixel slots in flight per thread (1 or 2; 0 = 1)
     int *ray_steps;              // optional: accepted steps per ray (not k_pair; single frame)
     int emission;                // 1 = some frame has plasma emission (the kernels with emission.cuh)
+    int lanes;                   // k_ham: lanes of a warp that take work items (0: all; launch_ham sets it)
     int sample_items;            // k_ham: 1 = a work item is a ray, not a pixel: colours of frames with several samples go
                                  // to sample_rgb (launch_combine follows)
     int hamiltonian;             // PRR_HAM_FP32 | PRR_HAM_FP64 mask: renders that integrate (x, p) in Hamiltonian form (k_ham.cu)
