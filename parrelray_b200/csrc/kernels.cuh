@@ -126,8 +126,10 @@ size_t adjoint_checkpoint_bytes(int precision);
 size_t adjoint_state_bytes(int precision);  // stored per thread and accepted step of a window
 int adjoint_blocks_per_sm(int precision);   // resident 128-thread CTAs of k_adjoint per SM
 // Accepted steps a thread stores (its window): longer rays recompute the earlier windows from checkpoints.  Most rays
-// of a frame take 1200 to 1400 steps (r + rout in steps of hmax), those that end on a sphere 1000 to 1500 more.
-constexpr int ADJ_WINDOW = 2048;
+// of a frame take 1200 to 1400 steps (r + rout in steps of hmax), those that end on a sphere 1000 to 1500 more. The
+// latter hold a gradient up (their one chain of dependent steps is its tail), so the window covers them: with 2048 they
+// ran their forward steps twice, 512x512 41.9 -> 39.0 ms, 256x256 30.9 -> 26.3, 160x120x4 with FP64 steps 32.6 -> 25.8.
+constexpr int ADJ_WINDOW = 4096;
 constexpr int ADJ_WINDOW_MIN = 64;  // the window shrinks to this when device memory is short
 
 // fma_peak.cu

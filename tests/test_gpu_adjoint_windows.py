@@ -1,4 +1,4 @@
-"""The adjoint's stored windows (parrelray_b200/csrc/k_adjoint.cu: 2048 accepted steps per ray, earlier windows
+"""The adjoint's stored windows (parrelray_b200/csrc/k_adjoint.cu: 4096 accepted steps per ray, earlier windows
 recomputed from checkpoints) and its warp-wide reverse sweep, against the FP64 host gradient with the bars of
 test_gpu_adjoint.py: rays of one window, of a window and a few steps, of several windows; ray counts that are not
 a multiple of a warp."""
