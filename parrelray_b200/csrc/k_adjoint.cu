@@ -30,9 +30,9 @@
 // and a fixed assignment of rays to threads cost 117 ms, without them 59 ms,
 // and with the closed forms of geod_vjp.cuh 37 ms (256x256 with FP64 steps:
 // 64.7, 41.5, 31.5 and, with adj_attempt's rule, 27.4 ms); windows of 4096
-// steps, which hold the longest rays (kernels.cuh), took 5 ms more off both.  The states are 36 bytes per FP32 step, 11 GB
-// written and read per 512x512 gradient: 3.4 ms of HBM time spread under the
-// arithmetic.
+// steps, which hold the longest rays (kernels.cuh), took 3 and 6 ms more off.
+// The states are 36 bytes per FP32 step, 11 GB written and read per 512x512
+// gradient: 3.4 ms of HBM time spread under the arithmetic.
 #include <cub/device/device_radix_sort.cuh>
 
 #include "dual.cuh"

@@ -26,10 +26,12 @@
 // scene/sphere.h:34-64), l < 1000 and the max_steps caps.  Initial data are
 // phys_init's null u, lowered once: p = g u.
 //
-// Scheduling is k_pair's (k_pair.cu): persistent CTAs, each lane owns one
-// pixel and integrates its SSAA samples in order with the RMS combine in
-// registers, one attempt per loop iteration, warp-aggregated refill of the
-// lanes whose pixel is complete every compaction_interval attempts.  The
+// Scheduling is k_pair's (k_pair.cu): persistent CTAs, warp-aggregated refill
+// of the lanes whose work item is complete every compaction_interval attempts.
+// An item is a ray of a frame with several samples (sample_items; its colour
+// goes to sample_rgb) or a pixel, whose SSAA samples a lane integrates in order
+// with the RMS combine in registers.  Attempts far from everything run in a row
+// (ham_attempts), the others pass the general accept step one by one.  The
 // three coordinate pairs (x, y), (p_x, p_y) and (z, p_z) share Blackwell's
 // paired FP32 instructions in the stage combinations, and the x/y twins of
 // the right-hand side (gradients, l, the gradient of Lam, the derivatives)
@@ -38,8 +40,8 @@
 // SPLIT (split precision): per-sample colours go to sample_rgb (the per-pixel
 // combine runs after the FP64 pass), and rays near a photon orbit
 // (near_critical on the initial data) or that dip below fp64_rfac * r_+ are
-// queued for k_fp64_requeue (k_persistent.cu), which integrates them again
-// from the camera in FP64, as for k_pair's split pass.
+// queued for k_ham_requeue (or, without PRR_HAM_FP64, k_fp64_requeue in
+// k_persistent.cu), which integrates them again from the camera in FP64.
 //
 // EMIS: the emission of emission.cuh at every accepted step, in its momentum
 // form (emis_step_p: k.u_e = p_mu u_e^mu, no lowering needed).
