@@ -281,7 +281,10 @@ prr_status prr_upload_plasma(prr_ctx *ctx, const prr_plasma_desc *plasma);
  * frame, each width*height pixels, row-major:
  *   out_rgb8: 3 bytes/pixel, round(255*x) (cudamaths/image.cu:31), may be NULL
  *   out_rgbf: 3 floats/pixel, the combined (and FXAA'd) colour, may be NULL
- * Synchronous; host buffers. */
+ * Synchronous; host buffers.  The context keeps its device scratch between
+ * calls: 12 bytes per pixel, 3 or 15 for the outputs, and 12 per ray (at most
+ * 3.2 GB) for frames with several samples where that is at most a quarter of
+ * the free memory. */
 prr_status prr_render(prr_ctx *ctx, const prr_frame_desc *frames, int n,
                       uint8_t *out_rgb8, float *out_rgbf, prr_stats *stats);
 
@@ -325,7 +328,15 @@ prr_status prr_trace_rays_f64(prr_ctx *ctx, const prr_frame_desc *frame,
  * kernel, stats->trace_ms the forward render time, stats->accepted the
  * adjoint's forward steps and stats->n_math_error the rays it dropped (their
  * checkpoints did not fit max_steps, or a recomputed segment disagreed with
- * the forward steps; neither happens on valid frames). */
+ * the forward steps; neither happens on valid frames).
+ * Device memory: every thread of one resident wave (up to 57 000 for FP32
+ * steps, 38 000 for FP64 steps) stores the states of a window of accepted
+ * steps, 36 bytes each (72 with FP64 steps), and a checkpoint per earlier
+ * window, whose steps are recomputed.  The window is 4096 steps (8.4 and
+ * 11 GB) where that is at most a quarter of the free memory, and shorter
+ * otherwise, down to under 1 GB; PRR_OPT_ADJOINT_WINDOW sets it.  The context
+ * keeps these buffers for its next gradient and gives them back when it runs
+ * short of memory itself, or in prr_destroy. */
 prr_status prr_adjoint(prr_ctx *ctx, const prr_frame_desc *frame, const float *dL_dimage, int sphere_index,
                        double grads[5], prr_stats *stats);
 
@@ -443,6 +454,9 @@ prr_status prr_autotune(prr_ctx *ctx, const prr_frame_desc *frame, prr_launch_co
                                      hooks and colours; in the Hamiltonian form the coordinate time is not
                                      integrated, so r.w of prr_trace_rays(_f64) is 0 there.  PRR_HAM_FP64
                                      also covers the FP64 pass of SPLIT; the adjoint always steps (x, u) */
+#define PRR_OPT_ADJOINT_WINDOW 4  /* accepted steps a thread of prr_adjoint stores (see there): 1 .. 1048576;
+                                     0 (default): chosen from the free device memory.  Gradients do not
+                                     depend on it */
 #define PRR_HAM_FP32 1
 #define PRR_HAM_FP64 2
 prr_status prr_set_option(prr_ctx *ctx, int option, long long value);

@@ -211,7 +211,7 @@ prr_status prr_upload_texture(prr_ctx *ctx, int id, const uint8_t *rgba8, int w,
     PRR_CK(ctx, cudaSetDevice(ctx->device));
     TexSlot &t = ctx->tex[id];
     size_t bytes = (size_t)w * h * 4;
-    if (t.buf.ensure(bytes) != PRR_OK) { fail(ctx, "prr_upload_texture: out of device memory"); return PRR_ERR_NOMEM; }
+    if (ensure_or_release(ctx, t.buf, bytes) != PRR_OK) { fail(ctx, "prr_upload_texture: out of device memory"); return PRR_ERR_NOMEM; }
     PRR_CK(ctx, cudaMemcpyAsync(t.buf.p, rgba8, bytes, cudaMemcpyHostToDevice, ctx->stream));
     PRR_CK(ctx, cudaStreamSynchronize(ctx->stream));
     t.w = w; t.h = h;
@@ -251,8 +251,8 @@ prr_status prr_upload_plasma(prr_ctx *ctx, const prr_plasma_desc *pd)
     PlasmaGrid &G = ctx->plasma;
     G.present = false;
     const size_t fb = (size_t)nn * sizeof(float);
-    if (G.n.ensure(fb) != PRR_OK || (pd->temperature && G.theta.ensure(fb) != PRR_OK) ||
-        (pd->velocity && G.vel.ensure((size_t)nn * sizeof(float4)) != PRR_OK)) {
+    if (ensure_or_release(ctx, G.n, fb) != PRR_OK || (pd->temperature && ensure_or_release(ctx, G.theta, fb) != PRR_OK) ||
+        (pd->velocity && ensure_or_release(ctx, G.vel, (size_t)nn * sizeof(float4)) != PRR_OK)) {
         fail(ctx, "prr_upload_plasma: out of device memory");
         return PRR_ERR_NOMEM;
     }
@@ -310,6 +310,10 @@ prr_status prr_set_option(prr_ctx *ctx, int option, long long value)
         }
         ctx->hamiltonian = (int)value;
         return PRR_OK;
+    case PRR_OPT_ADJOINT_WINDOW:
+        if (value < 0 || value > (1 << 20)) { ctx->err = "PRR_OPT_ADJOINT_WINDOW takes 0 (chosen) or 1 .. 1048576 steps"; return PRR_ERR_INVALID; }
+        ctx->adj_window = (int)value;
+        return PRR_OK;
     case PRR_OPT_WATCHDOG_CYCLES: ctx->watchdog_cycles = value > 0 ? value : 0; return PRR_OK;
     default: fail(ctx, "prr_set_option: unknown option"); return PRR_ERR_INVALID;
     }
@@ -323,7 +327,7 @@ prr_status prr_render(prr_ctx *ctx, const prr_frame_desc *frames, int n, uint8_t
     if (s != PRR_OK) return s;
     PRR_CK(ctx, cudaSetDevice(ctx->device));
     size_t npx = (size_t)plan.total_pixels;
-    if (ctx->out_u8.ensure(npx * 3) != PRR_OK || ctx->out_f.ensure(npx * 3 * sizeof(float)) != PRR_OK) {
+    if (ensure_or_release(ctx, ctx->out_u8, npx * 3) != PRR_OK || ensure_or_release(ctx, ctx->out_f, npx * 3 * sizeof(float)) != PRR_OK) {
         fail(ctx, "prr_render: out of device memory for outputs");
         return PRR_ERR_NOMEM;
     }
@@ -382,7 +386,7 @@ prr_status prr_measure_peak(prr_ctx *ctx, double *fp32_tflops, double *fp64_tflo
 {
     if (!ctx) return PRR_ERR_INVALID;
     PRR_CK(ctx, cudaSetDevice(ctx->device));
-    if (ctx->scratch.ensure(4096 * sizeof(double)) != PRR_OK) return PRR_ERR_NOMEM;
+    if (ensure_or_release(ctx, ctx->scratch, 4096 * sizeof(double)) != PRR_OK) return PRR_ERR_NOMEM;
     const int threads = 256, blocks = ctx->nsm * 8;
     for (int pass = 0; pass < 2; pass++) {
         double *outp = pass == 0 ? fp32_tflops : fp64_tflops;
@@ -413,7 +417,7 @@ prr_status prr_check_recip(prr_ctx *ctx, const double *x, int n, double *out)
         return PRR_ERR_INVALID;
     }
     PRR_CK(ctx, cudaSetDevice(ctx->device));
-    if (ctx->scratch.ensure((size_t)n * 5 * sizeof(double)) != PRR_OK) return PRR_ERR_NOMEM;
+    if (ensure_or_release(ctx, ctx->scratch, (size_t)n * 5 * sizeof(double)) != PRR_OK) return PRR_ERR_NOMEM;
     double *d_x = (double *)ctx->scratch.p, *d_out = d_x + n;
     PRR_CK(ctx, cudaMemcpyAsync(d_x, x, (size_t)n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     PRR_CK(ctx, launch_check_recip(d_x, n, d_out, ctx->stream));

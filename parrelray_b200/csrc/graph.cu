@@ -54,7 +54,7 @@ namespace {
 
 prr_status galloc(prr_graph *g, DevBuf &b, size_t bytes, const char *what)
 {
-    if (b.ensure(bytes) != PRR_OK) {
+    if (ensure_or_release(g->ctx, b, bytes) != PRR_OK) {
         g->ctx->err = std::string("prr_graph: out of device memory for ") + what + " (" + std::to_string(bytes) + " bytes)";
         return PRR_ERR_NOMEM;
     }
@@ -179,10 +179,8 @@ extern "C" prr_status prr_graph_create(prr_ctx *ctx, const prr_frame_desc *frame
         release(g); delete g; return s;
     }
     g->sample_items = wants_sample_items(ctx, plan, g->cfg);
-    if (g->sample_items && g->sample_rgb.ensure((size_t)plan.total_rays * 3 * sizeof(float)) != PRR_OK) {
-        cudaGetLastError();  // short of device memory: pixels as work items (SPLIT fails just below)
-        g->sample_items = false;
-    }
+    if (g->sample_items && plan.precision != PRR_PREC_SPLIT && !ensure_spare(g->sample_rgb, (size_t)plan.total_rays * 3 * sizeof(float)))
+        g->sample_items = false;  // short of device memory: pixels as work items
     if (plan.precision == PRR_PREC_SPLIT &&
         ((s = galloc(g, g->sample_rgb, (size_t)plan.total_rays * 3 * sizeof(float), "per-sample colours")) != PRR_OK ||
          (s = galloc(g, g->queue, (size_t)plan.total_rays * sizeof(unsigned long long), "FP64 queue")) != PRR_OK)) {

@@ -527,6 +527,17 @@ size_t adjoint_checkpoint_bytes(int precision)
 
 size_t adjoint_state_bytes(int precision) { return ADJ_STATE * (precision == PRR_PREC_FP32 ? sizeof(float) : sizeof(double)); }
 
+int adjoint_window(size_t budget, int threads, int max_steps, int precision)
+{
+    auto bytes = [&](int cap) {
+        return (size_t)threads * (cap * adjoint_state_bytes(precision) + (max_steps / cap + 2) * adjoint_checkpoint_bytes(precision));
+    };
+    int cap = ADJ_WINDOW;
+    while (cap > ADJ_WINDOW_MIN && cap / 2 >= max_steps) cap /= 2;
+    while (cap > ADJ_WINDOW_MIN && bytes(cap) > budget && bytes(cap / 2) < bytes(cap)) cap /= 2;
+    return cap;
+}
+
 int adjoint_blocks_per_sm(int precision)
 {
     int n = 0;

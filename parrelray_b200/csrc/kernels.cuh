@@ -130,7 +130,10 @@ int adjoint_blocks_per_sm(int precision);   // resident 128-thread CTAs of k_adj
 // latter hold a gradient up (their one chain of dependent steps is its tail), so the window covers them: with 2048 they
 // ran their forward steps twice, 512x512 41.9 -> 39.0 ms, 256x256 30.9 -> 26.3, 160x120x4 with FP64 steps 32.6 -> 25.8.
 constexpr int ADJ_WINDOW = 4096;
-constexpr int ADJ_WINDOW_MIN = 64;  // the window shrinks to this when device memory is short
+constexpr int ADJ_WINDOW_MIN = 64;
+// The longest window (ADJ_WINDOW halved, no longer than max_steps asks for) whose states and checkpoints take at most
+// `budget` bytes; where none does, the one that takes least (a shorter window has fewer states and more checkpoints).
+int adjoint_window(size_t budget, int threads, int max_steps, int precision);
 
 // fma_peak.cu
 cudaError_t launch_fma_peak(float *sink, int blocks, int threads, int iters, cudaStream_t st);

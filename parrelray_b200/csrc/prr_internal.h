@@ -57,6 +57,7 @@ struct prr_ctx {
     int hamiltonian = PRR_HAM_FP32 | PRR_HAM_FP64;  // renders in Hamiltonian form (PRR_OPT_HAMILTONIAN)
     long long watchdog_cycles = 0;
     std::vector<MetricPlugin> plugins;
+    int adj_window = 0;            // PRR_OPT_ADJOINT_WINDOW (0: adjoint_window chooses)
     int *ray_steps_out = nullptr;  // set by prr_adjoint around its forward render: per-ray accepted steps
     int last_launches = 0;
     float last_ms = 0.f;
@@ -103,6 +104,14 @@ prr_status trace_plan(prr_ctx *ctx, const RenderPlan &plan, float *h_state, doub
 prr_status collect_stats(prr_ctx *ctx, const RenderPlan &plan, prr_stats *stats);
 // Do the work items of a persistent launch of this plan under `cfg` be rays (k_ham's sample_items) rather than pixels?
 bool wants_sample_items(const prr_ctx *ctx, const RenderPlan &plan, const prr_launch_config &cfg);
+// DevBuf::ensure; short of device memory, the context first gives back the windows it keeps for its next gradient
+// (nothing uses them between prr_adjoint calls, which wait for their kernels).
+prr_status ensure_or_release(prr_ctx *ctx, DevBuf &b, size_t bytes);
+// Device bytes that scratch without which a call can do may take: a quarter of what is free with the `held` bytes it
+// would replace, so that other allocations of the process still succeed; never less than what is held.
+size_t spare_bytes(size_t held);
+// Grows `b` when that takes no more than spare_bytes; false (and `b` as it was, or empty) otherwise.
+bool ensure_spare(DevBuf &b, size_t bytes);
 // Resident CTAs per SM of the persistent kernel under the context's launch
 // configuration (its blocks_per_sm, or the occupancy limit when that is 0).
 int resolve_bpsm(prr_ctx *ctx, int precision, bool emission = false);

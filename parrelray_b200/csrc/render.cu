@@ -44,7 +44,7 @@ DevTex dev_tex(prr_ctx *ctx, int id)
 
 prr_status alloc(prr_ctx *ctx, DevBuf &b, size_t bytes, const char *what)
 {
-    if (b.ensure(bytes) != PRR_OK) {
+    if (ensure_or_release(ctx, b, bytes) != PRR_OK) {
         ctx->err = std::string("out of device memory for ") + what + " (" + std::to_string(bytes) + " bytes)";
         return PRR_ERR_NOMEM;
     }
@@ -117,6 +117,34 @@ prr_status emission_params(prr_ctx *ctx, int f, const prr_frame_desc &d, EmisPar
 }
 
 }  // namespace
+
+prr_status ensure_or_release(prr_ctx *ctx, DevBuf &b, size_t bytes)
+{
+    if (b.ensure(bytes) == PRR_OK) return PRR_OK;
+    cudaGetLastError();  // the failed allocation's, so the launches that follow do not report it
+    if (!ctx->adj_states.p && !ctx->adj_ckpt.p) return PRR_ERR_NOMEM;
+    ctx->adj_states.release();
+    ctx->adj_ckpt.release();
+    const prr_status s = b.ensure(bytes);
+    if (s != PRR_OK) cudaGetLastError();
+    return s;
+}
+
+size_t spare_bytes(size_t held)
+{
+    size_t free_b = 0, total = 0;
+    if (cudaMemGetInfo(&free_b, &total) != cudaSuccess) { cudaGetLastError(); return held; }
+    return std::max(held, (free_b + held) / 4);
+}
+
+bool ensure_spare(DevBuf &b, size_t bytes)
+{
+    if (b.cap >= bytes) return true;
+    if (bytes > spare_bytes(b.cap)) return false;
+    if (b.ensure(bytes) == PRR_OK) return true;
+    cudaGetLastError();
+    return false;
+}
 
 int resolve_bpsm(prr_ctx *ctx, int precision, bool emission)
 {
@@ -331,16 +359,14 @@ prr_status run_plan(prr_ctx *ctx, const RenderPlan &plan, uint8_t *d_rgb8, float
     if (s != PRR_OK) return s;
     const bool persistent = plan.mode != PRR_MODE_REFERENCE && ctx->schedule != PRR_SCHED_PLAIN && !plan.plugin;
     bool sample_items = persistent && wants_sample_items(ctx, plan, ctx->cfg);
-    if (sample_items && plan.precision != PRR_PREC_SPLIT && ctx->sample_rgb.ensure((size_t)plan.total_rays * 3 * sizeof(float)) != PRR_OK) {
-        cudaGetLastError();  // short of device memory: pixels as work items need no per-sample colours
-        sample_items = false;
-    }
+    if ((s = alloc(ctx, ctx->image, (size_t)plan.total_pixels * 3 * sizeof(float), "image")) != PRR_OK) return s;
+    if (sample_items && plan.precision != PRR_PREC_SPLIT && !ensure_spare(ctx->sample_rgb, (size_t)plan.total_rays * 3 * sizeof(float)))
+        sample_items = false;  // short of device memory: pixels as work items need no per-sample colours
     s = upload_plan(ctx, plan, st, sample_items);
     if (s != PRR_OK) return s;
     const int n = (int)plan.fp.size();
     unsigned long long *counters = (unsigned long long *)ctx->counters.p;
     int launches = 0;
-    if ((s = alloc(ctx, ctx->image, (size_t)plan.total_pixels * 3 * sizeof(float), "image")) != PRR_OK) return s;
     float *image = (float *)ctx->image.p;
     if (timed) PRR_CK(ctx, cudaEventRecord(ctx->e0, st));
     const FrameParams *d_fp = (const FrameParams *)ctx->frames.p;
@@ -637,18 +663,26 @@ extern "C" prr_status prr_adjoint(prr_ctx *ctx, const prr_frame_desc *frame, con
         ap.phase = std::atan2((double)S.center[1], (double)S.center[0]);
         ap.sph_z = S.center[2];
     }
-    // one resident wave, or fewer threads when there are fewer rays
-    const int threads = (int)std::min<long long>((long long)ctx->nsm * adjoint_blocks_per_sm(prec) * 128, (nrays + 127) / 128 * 128);
-    int cap = ADJ_WINDOW;
-    while (cap > ADJ_WINDOW_MIN && cap / 2 >= d.max_steps) cap /= 2;
-    while (ctx->adj_states.ensure((size_t)threads * cap * adjoint_state_bytes(prec)) != PRR_OK) {
-        cudaGetLastError();  // the failed allocation's, so the launches below do not report it
-        if (cap == ADJ_WINDOW_MIN) { ctx->err = "out of device memory for adjoint states"; return PRR_ERR_NOMEM; }
-        cap /= 2;
-    }
-    const int max_ckpt = d.max_steps / cap + 2;
-    if ((s = alloc(ctx, ctx->adj_ckpt, (size_t)threads * max_ckpt * adjoint_checkpoint_bytes(prec), "adjoint checkpoints")) != PRR_OK) return s;
     if ((s = alloc(ctx, ctx->adj_dl, (size_t)npx * 3 * sizeof(float) + 8 * sizeof(double), "adjoint inputs")) != PRR_OK) return s;
+    // one resident wave, or fewer threads when there are fewer rays
+    int threads = (int)std::min<long long>((long long)ctx->nsm * adjoint_blocks_per_sm(prec) * 128, (nrays + 127) / 128 * 128);
+    // The states of a window and the checkpoints of the earlier ones are sized together: a quarter of the free memory at
+    // most (or what the context holds already), then, where that cannot be had, the smallest pair, then fewer threads.
+    size_t spare = spare_bytes(ctx->adj_states.cap + ctx->adj_ckpt.cap);
+    int cap = 0, max_ckpt = 0;
+    while (true) {
+        cap = ctx->adj_window ? ctx->adj_window : adjoint_window(spare, threads, d.max_steps, prec);
+        max_ckpt = d.max_steps / cap + 2;
+        if (ctx->adj_states.ensure((size_t)threads * cap * adjoint_state_bytes(prec)) == PRR_OK &&
+            ctx->adj_ckpt.ensure((size_t)threads * max_ckpt * adjoint_checkpoint_bytes(prec)) == PRR_OK)
+            break;
+        cudaGetLastError();  // the failed allocation's
+        ctx->adj_states.release();
+        ctx->adj_ckpt.release();
+        if (spare) spare = 0;
+        else if (threads > 128) threads = std::max(128, threads / 256 * 128);
+        else { ctx->err = "out of device memory for adjoint states"; return PRR_ERR_NOMEM; }
+    }
     float *d_dl = (float *)ctx->adj_dl.p;
     double *d_grad = (double *)((char *)ctx->adj_dl.p + ((size_t)npx * 3 * sizeof(float) + 7) / 8 * 8);
     cudaStream_t st = ctx->stream;
