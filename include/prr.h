@@ -435,6 +435,10 @@ prr_status prr_load_metric_plugin(prr_ctx *ctx, const char *path, int *metric_id
 
 /* ---- scheduler tuning (new) ---- */
 prr_status prr_set_schedule(prr_ctx *ctx, int schedule, const prr_launch_config *cfg);
+/* The context's launch shape.  Before prr_set_schedule or prr_autotune sets
+ * one it is the Hamiltonian renderer's (PRR_OPT_HAMILTONIAN); the other
+ * renderers then run 128-thread CTAs where those are faster, and
+ * prr_graph_get_launch_config says what a graph recorded. */
 prr_status prr_get_launch_config(prr_ctx *ctx, prr_launch_config *cfg);
 /* Times candidate launch shapes on `frame` and keeps the fastest. */
 prr_status prr_autotune(prr_ctx *ctx, const prr_frame_desc *frame, prr_launch_config *best);

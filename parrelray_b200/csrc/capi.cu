@@ -134,7 +134,8 @@ prr_status prr_create(int device, prr_ctx **out)
         delete ctx;
         return PRR_ERR_CUDA;
     }
-    // The launch shape of a context that was not tuned: the one prr_autotune settles on for full-size frames.  Against
+    // The launch shape of a context that was not tuned: the one prr_autotune settles on for full-size frames of k_ham (the
+    // other renderers' CTA size: render.cu:launch_shape).  Against
     // 128-thread CTAs refilled after every attempt (what it was): 1920x1080x4 Kerr frame 257 -> 170 ms, FP64 960x540
     // 33 -> 21 ms, split batch 114 -> 70 ms, 640x360x9 56 -> 43 ms, disk 640x640 14.5 -> 12.0 ms; a 320x180 frame, which
     // does not fill the chip, 2.4 -> 2.5 ms.
@@ -286,6 +287,7 @@ prr_status prr_set_schedule(prr_ctx *ctx, int schedule, const prr_launch_config 
             return PRR_ERR_INVALID;
         }
         ctx->cfg = *cfg;
+        ctx->shape_set = true;
     }
     ctx->schedule = schedule;
     return PRR_OK;

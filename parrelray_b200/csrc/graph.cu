@@ -170,8 +170,8 @@ extern "C" prr_status prr_graph_create(prr_ctx *ctx, const prr_frame_desc *frame
     const size_t nf = plan.fp.size();
     g->d_rgb8 = d_rgb8;
     g->d_rgbf = d_rgbf;
-    g->cfg = ctx->cfg;
-    g->bpsm = resolve_bpsm(ctx, plan.precision, plan.any_emission);
+    g->cfg = launch_shape(ctx, plan.precision, plan.any_emission, plan.total_pixels);
+    g->bpsm = resolve_bpsm(ctx, g->cfg, plan.precision, plan.any_emission);
     if ((s = galloc(g, g->frames, nf * sizeof(FrameParams), "frame parameters")) != PRR_OK ||
         (s = galloc(g, g->frame_begin, (nf + 1) * sizeof(long long), "frame table")) != PRR_OK ||
         (s = galloc(g, g->counters, C_COUNT * sizeof(unsigned long long), "counters")) != PRR_OK ||

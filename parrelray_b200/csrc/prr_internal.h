@@ -53,6 +53,7 @@ struct prr_ctx {
     PlasmaGrid plasma;
     int schedule = PRR_SCHED_PERSISTENT;
     prr_launch_config cfg{};
+    bool shape_set = false;  // cfg is the caller's (prr_set_schedule) or prr_autotune's, not prr_create's
     int geod_table = -1;  // -1: per schedule (PERSISTENT contraction, PLAIN table); 0: contraction; 1: table
     int hamiltonian = PRR_HAM_FP32 | PRR_HAM_FP64;  // renders in Hamiltonian form (PRR_OPT_HAMILTONIAN)
     long long watchdog_cycles = 0;
@@ -112,6 +113,7 @@ prr_status ensure_or_release(prr_ctx *ctx, DevBuf &b, size_t bytes);
 size_t spare_bytes(size_t held);
 // Grows `b` when that takes no more than spare_bytes; false (and `b` as it was, or empty) otherwise.
 bool ensure_spare(DevBuf &b, size_t bytes);
-// Resident CTAs per SM of the persistent kernel under the context's launch
-// configuration (its blocks_per_sm, or the occupancy limit when that is 0).
-int resolve_bpsm(prr_ctx *ctx, int precision, bool emission = false);
+// The launch shape of a persistent render of `items` pixels: the context's, with the CTA size of the kernel where nobody set one.
+prr_launch_config launch_shape(const prr_ctx *ctx, int precision, bool emission, long long items);
+// Resident CTAs per SM of the persistent kernel under `cfg` (its blocks_per_sm, or the occupancy limit when that is 0).
+int resolve_bpsm(const prr_ctx *ctx, const prr_launch_config &cfg, int precision, bool emission);

@@ -146,11 +146,25 @@ bool ensure_spare(DevBuf &b, size_t bytes)
     return false;
 }
 
-int resolve_bpsm(prr_ctx *ctx, int precision, bool emission)
+// A context's shape before anyone sets one is k_ham's (prr_create).  The (x, u) renderers run 128-thread CTAs in FP64, and
+// in FP32 without the table up to 2048 work items per SM: their 64-thread instantiations hold more CTAs in fewer registers,
+// which costs a ray its latency, and only a launch of several items per lane has other rays to cover it.  Medians, 64
+// and 128 threads: FP64 96x54 11.9 and 10.9 ms, 320x180 16.7 and 13.7, 960x540 89.7 and 83.3, 640x360 with emission
+// 46.1 and 45.2; FP32 320x180 6.41 and 5.97, 500x281 9.88 and 8.95, 640x360 12.80 and 12.55, 800x450 24.8 and 27.1,
+// 960x540 33.0 and 33.9; the table form 320x180 32.1 and 33.3, 960x540 197 and 222.
+prr_launch_config launch_shape(const prr_ctx *ctx, int precision, bool emission, long long items)
 {
-    if (ctx->cfg.blocks_per_sm > 0) return ctx->cfg.blocks_per_sm;
-    int b = persistent_occupancy(precision, ctx->geod_table == 1, ctx->cfg.block_size, ctx->cfg.rays_per_thread, emission,
-                                 ctx->hamiltonian);
+    prr_launch_config c = ctx->cfg;
+    if (ctx->shape_set || renders_with_ham(precision, ctx->geod_table == 1, ctx->hamiltonian, c.rays_per_thread, emission)) return c;
+    const bool table = ctx->geod_table == 1 && precision == PRR_PREC_FP32;
+    if (precision == PRR_PREC_FP64 || (!table && items <= 2048ll * ctx->nsm)) c.block_size = 128;
+    return c;
+}
+
+int resolve_bpsm(const prr_ctx *ctx, const prr_launch_config &cfg, int precision, bool emission)
+{
+    if (cfg.blocks_per_sm > 0) return cfg.blocks_per_sm;
+    int b = persistent_occupancy(precision, ctx->geod_table == 1, cfg.block_size, cfg.rays_per_thread, emission, ctx->hamiltonian);
     return b > 0 ? b : 1;
 }
 
@@ -322,7 +336,7 @@ static prr_status upload_plan(prr_ctx *ctx, const RenderPlan &plan, cudaStream_t
     return PRR_OK;
 }
 
-static PersistentArgs persistent_args(prr_ctx *ctx, const RenderPlan &plan, bool sample_items)
+static PersistentArgs persistent_args(prr_ctx *ctx, const RenderPlan &plan, const prr_launch_config &cfg, bool sample_items)
 {
     PersistentArgs a;
     memset(&a, 0, sizeof(a));
@@ -334,9 +348,9 @@ static PersistentArgs persistent_args(prr_ctx *ctx, const RenderPlan &plan, bool
     a.counters = (unsigned long long *)ctx->counters.p;
     a.geod_table = ctx->geod_table == 1;
     a.hamiltonian = ctx->hamiltonian;
-    a.compaction_interval = ctx->cfg.compaction_interval;
+    a.compaction_interval = cfg.compaction_interval;
     a.watchdog_cycles = ctx->watchdog_cycles;
-    a.rays_per_thread = ctx->cfg.rays_per_thread;
+    a.rays_per_thread = cfg.rays_per_thread;
     a.ray_steps = ctx->ray_steps_out;
     a.emission = plan.any_emission;
     return a;
@@ -358,7 +372,8 @@ prr_status run_plan(prr_ctx *ctx, const RenderPlan &plan, uint8_t *d_rgb8, float
     prr_status s = check_emission_schedule(ctx, plan);
     if (s != PRR_OK) return s;
     const bool persistent = plan.mode != PRR_MODE_REFERENCE && ctx->schedule != PRR_SCHED_PLAIN && !plan.plugin;
-    bool sample_items = persistent && wants_sample_items(ctx, plan, ctx->cfg);
+    const prr_launch_config cfg = launch_shape(ctx, plan.precision, plan.any_emission, plan.total_pixels);
+    bool sample_items = persistent && wants_sample_items(ctx, plan, cfg);
     if ((s = alloc(ctx, ctx->image, (size_t)plan.total_pixels * 3 * sizeof(float), "image")) != PRR_OK) return s;
     if (sample_items && plan.precision != PRR_PREC_SPLIT && !ensure_spare(ctx->sample_rgb, (size_t)plan.total_rays * 3 * sizeof(float)))
         sample_items = false;  // short of device memory: pixels as work items need no per-sample colours
@@ -414,9 +429,9 @@ prr_status run_plan(prr_ctx *ctx, const RenderPlan &plan, uint8_t *d_rgb8, float
         }
     } else {
         trace_timed = timed;
-        PersistentArgs a = persistent_args(ctx, plan, sample_items);
+        PersistentArgs a = persistent_args(ctx, plan, cfg, sample_items);
         a.image = image;
-        const int bpsm = resolve_bpsm(ctx, plan.precision, plan.any_emission);
+        const int bpsm = resolve_bpsm(ctx, cfg, plan.precision, plan.any_emission);
         if (plan.precision == PRR_PREC_SPLIT) {
             if ((s = alloc(ctx, ctx->sample_rgb, (size_t)plan.total_rays * 3 * sizeof(float), "per-sample colours")) != PRR_OK) return s;
             if ((s = alloc(ctx, ctx->queue, (size_t)plan.total_rays * sizeof(unsigned long long), "FP64 queue")) != PRR_OK) return s;
@@ -424,7 +439,7 @@ prr_status run_plan(prr_ctx *ctx, const RenderPlan &plan, uint8_t *d_rgb8, float
             a.fp64_queue = (unsigned long long *)ctx->queue.p;
             a.fp64_capacity = plan.total_rays;
             if (timed) PRR_CK(ctx, cudaEventRecord(ctx->t0, st));
-            PRR_CK(ctx, launch_persistent(a, PRR_PREC_SPLIT, ctx->cfg.block_size, bpsm, ctx->nsm, st));
+            PRR_CK(ctx, launch_persistent(a, PRR_PREC_SPLIT, cfg.block_size, bpsm, ctx->nsm, st));
             PRR_CK(ctx, launch_fp64_requeue(a, 128, ctx->nsm, st));
             if (timed) PRR_CK(ctx, cudaEventRecord(ctx->t1, st));
             launches += 2;
@@ -438,7 +453,7 @@ prr_status run_plan(prr_ctx *ctx, const RenderPlan &plan, uint8_t *d_rgb8, float
             a.rgb8 = d_rgb8;
             if (sample_items) a.sample_rgb = (float *)ctx->sample_rgb.p;
             if (timed) PRR_CK(ctx, cudaEventRecord(ctx->t0, st));
-            PRR_CK(ctx, launch_persistent(a, plan.precision, ctx->cfg.block_size, bpsm, ctx->nsm, st));
+            PRR_CK(ctx, launch_persistent(a, plan.precision, cfg.block_size, bpsm, ctx->nsm, st));
             if (timed) PRR_CK(ctx, cudaEventRecord(ctx->t1, st));
             launches++;
             for (int f = 0; f < n; f++) {
@@ -475,9 +490,10 @@ prr_status trace_plan(prr_ctx *ctx, const RenderPlan &plan, float *h_state, doub
     prr_status s = check_emission_schedule(ctx, plan);
     if (s != PRR_OK) return s;
     const int prec = plan.precision == PRR_PREC_FP64 ? PRR_PREC_FP64 : PRR_PREC_FP32;
+    const prr_launch_config cfg = launch_shape(ctx, prec, plan.any_emission, plan.total_pixels);
     const bool sample_items = plan.mode != PRR_MODE_REFERENCE && !plan.plugin && !(ctx->schedule == PRR_SCHED_PLAIN && !h_state64) &&
                               plan.any_ssaa && !plan.any_emission &&
-                              renders_with_ham(prec, ctx->geod_table == 1, ctx->hamiltonian, ctx->cfg.rays_per_thread, plan.any_emission);
+                              renders_with_ham(prec, ctx->geod_table == 1, ctx->hamiltonian, cfg.rays_per_thread, plan.any_emission);
     s = upload_plan(ctx, plan, st, sample_items);
     if (s != PRR_OK) return s;
     const FrameParams &p = plan.fp[0];
@@ -506,12 +522,12 @@ prr_status trace_plan(prr_ctx *ctx, const RenderPlan &plan, float *h_state, doub
         ctx->last_launches = launches;
     } else {
         if ((s = alloc(ctx, ctx->image, (size_t)plan.total_pixels * 3 * sizeof(float), "image")) != PRR_OK) return s;
-        PersistentArgs a = persistent_args(ctx, plan, sample_items);
+        PersistentArgs a = persistent_args(ctx, plan, cfg, sample_items);
         a.image = (float *)ctx->image.p;
         a.sample_rgb = rgb;
         if (h_state64) a.ray_state64 = (double *)ctx->state.p;
         else a.ray_state = (float *)ctx->state.p;
-        PRR_CK(ctx, launch_persistent(a, prec, ctx->cfg.block_size, resolve_bpsm(ctx, prec, plan.any_emission), ctx->nsm, st));
+        PRR_CK(ctx, launch_persistent(a, prec, cfg.block_size, resolve_bpsm(ctx, cfg, prec, plan.any_emission), ctx->nsm, st));
         ctx->last_launches = 1;
     }
     PRR_CK(ctx, cudaEventRecord(ctx->e1, st));
@@ -572,7 +588,9 @@ extern "C" prr_status prr_autotune(prr_ctx *ctx, const prr_frame_desc *frame, pr
     PRR_CK(ctx, cudaSetDevice(ctx->device));
     const prr_launch_config saved = ctx->cfg;
     const int saved_sched = ctx->schedule;
+    const bool saved_set = ctx->shape_set;
     ctx->schedule = PRR_SCHED_PERSISTENT;
+    ctx->shape_set = true;
     prr_launch_config winner = saved;
     float best_ms = 1e30f;
     // candidates: CTA size x refill interval x pixel slots per thread, each at the
@@ -595,7 +613,7 @@ extern "C" prr_status prr_autotune(prr_ctx *ctx, const prr_frame_desc *frame, pr
                 float ms = 1e30f;
                 for (int rep = 0; rep < 3; rep++) {
                     s = run_plan(ctx, plan, nullptr, nullptr, ctx->stream, true);
-                    if (s != PRR_OK) { ctx->cfg = saved; ctx->schedule = saved_sched; return s; }
+                    if (s != PRR_OK) { ctx->cfg = saved; ctx->schedule = saved_sched; ctx->shape_set = saved_set; return s; }
                     ms = std::min(ms, ctx->last_ms);
                     if (rep == 0 && ms > 1.1f * best_ms) break;
                 }
