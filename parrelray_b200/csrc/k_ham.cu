@@ -47,6 +47,7 @@
 // form (emis_step_p: k.u_e = p_mu u_e^mu, no lowering needed).
 #include "kernels.cuh"
 #include "phys_pair.cuh"
+#include "sphere_path.cuh"
 
 namespace prr {
 
@@ -367,37 +368,6 @@ template <class V> PRR_DEV void upd2(V &s, V &c, V v)
         s.x += v.x;
         s.y += v.y;
     }
-}
-
-// Path length within which a ray of intersection mode at p, flying along the unit vector v, cannot pass
-// Sphere::intersects on S with the window w (hmin): 0 when that cannot be said.  With rho = p - c, D = |rho|, b = -v.rho
-// and disc = b^2 - (D^2 - R^2), the test's distance is d = 2b - sqrt(disc), and a hit needs 0 <= d <= sqrt(w) (the
-// factor 2 lets a head-on ray fly on inside the sphere, down to D = R/2).  Along a path of curvature <= kappa, b falls
-// by at most (1 + D kappa) per length and disc changes by at most 2 D^2 kappa, so over a length S
-//     d >= 2 (b - S (1 + D kappa)) - sqrt(disc + 2 D^2 kappa S)
-// and, where the ray has passed (d < 0), d <= 2 (b + S D kappa) - sqrt(disc - 2 D^2 kappa S).  kappa <= 4M/r^2 for null geodesics in
-// Kerr-Schild coordinates at r >= 4M (maximum over 10^6 random states); 10 is used.  4e-6 D^2 under the root and 1e-5 D
-// outside it cover the FP32 rounding of the test.
-template <class T>
-PRR_DEV float sphere_path(const DevSphere &S, T px, T py, T pz, T vx, T vy, T vz, float w, float M, float r2)
-{
-    const float dx = (float)(px - (T)S.cx), dy = (float)(py - (T)S.cy), dz = (float)(pz - (T)S.cz);
-    const float D2 = fmaxf(dx * dx + dy * dy + dz * dz, 1e-30f), D = D2 * sfu_rsqrt(D2);
-    if (D > 1.1f * S.r + sqrtf(w)) return 0.9f * (D - 1.1f * S.r - sqrtf(w));  // far from it (R^2 + w/3 bounds a hit)
-    if (!(r2 >= 16.0f * M * M)) return 0.0f;
-    const float b = -((float)vx * dx + (float)vy * dy + (float)vz * dz);
-    const float disc = b * b - (D2 - S.r * S.r);
-    const float kap = r2 > 0.0f ? 10.0f * M * sfu_rcp(r2) : 0.0f, grow = 2.0f * D2 * kap, err = 4e-6f * D2;
-    const float sw = 1.00001f * sqrtf(w) + 1e-5f * D;
-    // ahead: half of the way that straight flight has left
-    const float S1 = 0.25f * (2.0f * b - sqrtf(fmaxf(disc, 0.0f) + err) - sw);
-    const float S1c = fminf(S1, 0.2f * D);
-    if (S1c > 0.0f && 2.0f * (b - S1c * (1.0f + D * kap)) - sqrtf(fmaxf(disc, 0.0f) + grow * S1c + err) > sw) return S1c;
-    // missing it, or passed: a fixed share of the size
-    const float S2 = 0.05f * D;
-    if (disc + grow * S2 + err < 0.0f) return S2;
-    if (2.0f * (b + D * kap * S2) - sqrtf(fmaxf(disc - grow * S2 - err, 0.0f)) < -1e-5f * D) return S2;
-    return 0.0f;
 }
 
 // phys_accept (phys_stepper.cuh) on the Hamiltonian state.
