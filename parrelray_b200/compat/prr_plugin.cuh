@@ -107,6 +107,15 @@ __device__ inline void from_ray(const Ray &T, RefRay &R)
     R.u = {T.u.x, T.u.y, T.u.z, T.u.w};
 }
 
+// REFERENCE mode calls one copy of the header's geodesic from its six stages: inlined at each of them, a geodesic through
+// a Christoffel table makes a loop that the instruction cache does not hold.  (PHYSICAL mode keeps it inlined: there
+// the compiler may contract its multiply-adds with the stages'.)
+#if PRR_PLUGIN_PART == 1
+#define PRR_GEOD_COPY __noinline__
+#else
+#define PRR_GEOD_COPY
+#endif
+
 // The header's functions as the solver's hook set (ref_stepper.cuh).  A
 // header written for SPHERICAL states (r, theta, phi, t) is compiled with
 // SPHERICAL defined, as the reference compiles it: its rays then start at
@@ -138,7 +147,7 @@ struct PluginHooks {
         mat4 m = getMetric(&T, space);
         for (int i = 0; i < 16; i++) g[i] = m.e[i];
     }
-    __device__ V4<float> geod(const V4<float> &x, const V4<float> &u) const
+    PRR_GEOD_COPY __device__ V4<float> geod(const V4<float> &x, const V4<float> &u) const
     {
         f4 d = getGeod(f4(x.x, x.y, x.z, x.w), f4(u.x, u.y, u.z, u.w), space);
         return {d.x, d.y, d.z, d.w};

@@ -8,7 +8,10 @@
 // error are evaluated only where they can decide something, and the sphere
 // test only near a sphere (ref_stepper.cuh): 1920x1080x4 Kerr frame at eps
 // 1e-3 813 -> 628 ms, 320x180x4 64 -> 51 ms, 320x180 Schwarzschild 13.8 ->
-// 11.3 ms, the same bits.
+// 11.3 ms, the same bits.  The Kerr geodesic has a kernel of its own: with
+// both geodesics in each of the six stages 320x180 with three spheres took
+// 40.1 ms (Schwarzschild 37.6, without spheres 6.0, Kerr 960x540x4 164), and
+// takes 33.7 (35.2, 5.6, 148) with one.
 #include "kernels.cuh"
 #include "ref_stepper.cuh"
 
@@ -22,6 +25,7 @@ __device__ __forceinline__ void warp_add(unsigned long long *p, unsigned long lo
     if ((threadIdx.x & 31) == (__ffs(mask) - 1)) atomicAdd(p, v);
 }
 
+template <bool KERR>
 __global__ void __launch_bounds__(128) k_ref_trace(const FrameParams *__restrict__ fps, int frame, long long nrays,
                                                    float *__restrict__ state, float *__restrict__ rgb,
                                                    unsigned long long *__restrict__ counters)
@@ -34,9 +38,10 @@ __global__ void __launch_bounds__(128) k_ref_trace(const FrameParams *__restrict
     int s = (int)(rid - pix * S);
     int x = (int)(pix % fp.width), y = (int)(pix / fp.width);
     RefRay R;
-    ref_init(fp, x, y, s, R);
-    if (fp.solver == PRR_SOLVER_EULER) ref_euler(fp, R);
-    else ref_rkf(fp, R);
+    const BuiltinHooks<KERR> hk{fp};
+    ref_init_h(fp, hk, x, y, s, R);
+    if (fp.solver == PRR_SOLVER_EULER) ref_euler_h(fp, hk, R);
+    else ref_rkf_h(fp, hk, R);
     V3<float> c = ray_colour<float>(fp, R.result, R.r, R.u);
     if (state) {
         float *o = state + 12 * rid;
@@ -60,15 +65,17 @@ __global__ void __launch_bounds__(128) k_ref_trace(const FrameParams *__restrict
     }
 }
 
-cudaError_t launch_ref_trace(const FrameParams *d_fp, int frame, long long nrays, float *state, float *rgb,
+cudaError_t launch_ref_trace(const FrameParams &fp, const FrameParams *d_fp, int frame, long long nrays, float *state, float *rgb,
                              unsigned long long *counters, cudaStream_t st)
 {
     if (nrays <= 0) return cudaSuccess;
     // a warp leaves when its longest ray does: one-warp CTAs free their slots at once, which a frame of about a wave
-    // likes (320x180: 11.3 ms against 11.8 with four warps), and a large one not (1920x1080x4: 636 and 628)
-    const int block = nrays <= (1 << 19) ? 32 : 128;
+    // likes (320x180: 11.3 ms against 11.8 with four warps), and a large one not (1920x1080x4: 636 and 628), nor one
+    // whose eps is so tight that rays take up to 10^6 attempts (96x54 at eps 1e-6: 4.78 s against 4.56)
+    const int block = ref_bounded(fp) && nrays <= (1 << 19) ? 32 : 128;
     long long grid = (nrays + block - 1) / block;
-    k_ref_trace<<<(unsigned)grid, block, 0, st>>>(d_fp, frame, nrays, state, rgb, counters);
+    auto k = fp.metric == PRR_METRIC_KERR ? k_ref_trace<true> : k_ref_trace<false>;
+    k<<<(unsigned)grid, block, 0, st>>>(d_fp, frame, nrays, state, rgb, counters);
     return cudaGetLastError();
 }
 

@@ -27,9 +27,9 @@ enum Counter {
 };
 
 // k_reference.cu: REFERENCE-mode tracing, one thread per ray of frame
-// `frame` (rays [0, nrays)).  state: 12 floats/ray, rgb: 3 floats/ray (either
+// `frame` (rays [0, nrays); fp is its d_fp[frame] on the host).  state: 12 floats/ray, rgb: 3 floats/ray (either
 // may be null).
-cudaError_t launch_ref_trace(const FrameParams *d_fp, int frame, long long nrays, float *state, float *rgb,
+cudaError_t launch_ref_trace(const FrameParams &fp, const FrameParams *d_fp, int frame, long long nrays, float *state, float *rgb,
                              unsigned long long *counters, cudaStream_t st);
 
 // post.cu: SSAA combine of per-sample colours into an FP32 image.

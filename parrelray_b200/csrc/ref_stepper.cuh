@@ -35,11 +35,12 @@ struct RefTab {
                            K54 = (float)(28561.0 / 56430.0), K55 = (float)(-9.0 / 50.0), K56 = (float)(2.0 / 55.0);
 };
 
-PRR_DEV V4<float> ref_geod(const FrameParams &fp, const V4<float> &x, const V4<float> &u)
+// KERR: the frame's metric is Kerr (one geodesic to a kernel: k_reference.cu)
+template <bool KERR> PRR_DEV V4<float> ref_geod(const FrameParams &fp, const V4<float> &x, const V4<float> &u)
 {
+    if constexpr (KERR) return geod_ks<float>(x, u, fp.M, fp.a);
     if (fp.metric == PRR_METRIC_FLAT) return {0.0f, 0.0f, 0.0f, 0.0f};
-    if (fp.metric == PRR_METRIC_SCHWARZSCHILD) return geod_schw_ref(x, u, fp.rs);
-    return geod_ks<float>(x, u, fp.M, fp.a);
+    return geod_schw_ref(x, u, fp.rs);
 }
 
 PRR_DEV bool isnan4(const V4<float> &a) { return isnan(a.x) || isnan(a.y) || isnan(a.z) || isnan(a.w); }
@@ -88,7 +89,8 @@ PRR_DEV void ref_metric(const FrameParams &fp, const RefRay &R, float g[16])
 }
 
 // Can Sphere::intersects pass on some sphere for a ray at p, with a window up to hmax?  (far2 bounds |p - c|^2 of a
-// hit, render.cu:build_plan; it covers hmax only, so a larger first step always tests.)
+// hit, render.cu:build_plan; it covers hmax only, so a larger first step always tests.)  A state that is not finite is no
+// hit in either place: the test's distance is NaN, which is not the nearest.
 PRR_DEV bool ref_near(const FrameParams &fp, const V4<float> &p)
 {
     bool near = fp.h > fp.hmax;
@@ -97,6 +99,24 @@ PRR_DEV bool ref_near(const FrameParams &fp, const V4<float> &p)
         near |= !(dx * dx + dy * dy + dz * dz > fp.sph[s].far2);
     }
     return near;
+}
+
+// Where a built-in metric's geodesic cannot overflow or divide by zero over the stages of a step: 1e-5 <= r <= 1e8, |u| <= 1e5
+// and h <= 1/4, with the stage points within r/16 or so of x (s = h U / r small).  False on NaN (a maximum passes it over).
+PRR_DEV bool ref_tame(float R2, float r2, const V4<float> &u, float h)
+{
+    return r2 >= 1e-10f && R2 <= 1e16f && fabsf(u.x) + fabsf(u.y) + fabsf(u.z) + fabsf(u.w) <= 1e5f && h <= 0.25f;
+}
+
+// Is the sixth stage of an intersection-mode step from (x, u) finite for certain?  (Its weight in the result is zero, but
+// 0 * NaN is NaN: elsewhere it is evaluated.)  With r >= 4M and s <= 1/256 the accelerations add less than a fifth to the stage
+// velocities, which h <= 1/4 lets grow to 1.8 U, so the stage points lie within 14 h U < r/16 of x.
+PRR_DEV bool ref_finite_stage(const FrameParams &fp, const V4<float> &x, const V4<float> &u, float h)
+{
+    const float U = fmaxf(fmaxf(fabsf(u.x), fabsf(u.y)), fmaxf(fabsf(u.z), fabsf(u.w)));
+    const float a = fp.metric == PRR_METRIC_KERR ? fp.a : 0.0f, M = fp.metric == PRR_METRIC_FLAT ? 0.0f : fp.M;
+    const float R2 = x.x * x.x + x.y * x.y + x.z * x.z, r2 = 0.999f * (R2 - a * a), hU = 256.0f * h * U;
+    return ref_tame(R2, r2, u, h) && r2 >= 16.1f * M * M && hU * hU <= r2;
 }
 
 // Is the error of a step h from (x, u) under half of eps whatever the sixth stage says?  With U the largest component
@@ -111,8 +131,11 @@ PRR_DEV bool ref_small_error(const FrameParams &fp, const V4<float> &x, const V4
     const float R2 = x.x * x.x + x.y * x.y + x.z * x.z, r2 = 0.999f * (R2 - a * a);  // under the Kerr-Schild r^2
     const float ir = sfu_rsqrt(r2), hU = h * U, s = hU * ir;
     const float X = sfu_rsqrt(R2) * R2 + fabsf(x.w) + U;
-    return r2 >= 16.1f * M * M && s <= 0.0625f && h <= 0.25f && hU * (0.01f * h + 0.2f * s * M * ir) + 7.2e-7f * X <= 0.5f * fp.eps;
+    return ref_tame(R2, r2, u, h) && r2 >= 16.1f * M * M && s <= 0.0625f && hU * (0.01f * h + 0.2f * s * M * ir) + 7.2e-7f * X <= 0.5f * fp.eps;
 }
+
+// Can ref_small_error hold anywhere?  Not where eps is so tight that the stages' own error or the sums' rounding leave no room.
+PRR_HD bool ref_bounded(const FrameParams &fp) { return 0.002f * fp.hmax * fp.hmax + 4e-5f <= 0.5f * fp.eps; }
 
 // User_UPDATE
 PRR_DEV bool ref_update(const FrameParams &fp, RefRay &R, float h)
@@ -134,13 +157,14 @@ PRR_DEV bool ref_endloop(const FrameParams &fp, RefRay &R, float th)
     return true;
 }
 
-struct BuiltinHooks {
+template <bool KERR> struct BuiltinHooks {
     static constexpr bool kSpherical = false;  // Cartesian (x, y, z, t) states
-    static constexpr bool kErrorBound = true;  // small_error holds for the metric (ref_small_error)
+    static constexpr bool kErrorBound = true;  // small_error and finite_stage hold for the metric
+    PRR_DEV bool finite_stage(const V4<float> &x, const V4<float> &u, float h) const { return ref_finite_stage(fp, x, u, h); }
     PRR_DEV bool small_error(const V4<float> &x, const V4<float> &u, float h) const { return ref_small_error(fp, x, u, h); }
     const FrameParams &fp;
     PRR_DEV void metric(const RefRay &R, float g[16]) const { ref_metric(fp, R, g); }
-    PRR_DEV V4<float> geod(const V4<float> &x, const V4<float> &u) const { return ref_geod(fp, x, u); }
+    PRR_DEV V4<float> geod(const V4<float> &x, const V4<float> &u) const { return ref_geod<KERR>(fp, x, u); }
     PRR_DEV bool loop(RefRay &) const { return true; }
     PRR_DEV bool update(RefRay &R, float h) const { return ref_update(fp, R, h); }
     PRR_DEV bool endloop(RefRay &R, float trace_h) const { return ref_endloop(fp, R, trace_h); }
@@ -154,8 +178,7 @@ template <class H> PRR_DEV void ref_rkf_h(const FrameParams &fp, const H &hk, Re
     float h = fp.h, hmin = fp.hmin, hmax = fp.hmax, _h = h, eps = fp.eps, trace_h = fp.h;
     V4<float> x = R.r, u = R.u, _x = x, _u = u, __x, __u;
     bool intersect = false;
-    // eps so tight that the stages' own error or the sums' rounding leave no room: do not look (ref_small_error)
-    const bool bounded = 0.002f * hmax * hmax + 4e-5f <= 0.5f * eps;
+    const bool bounded = ref_bounded(fp);
     int i = 0;
     for (float l = 0.0f; l < 1000.0f;) {
         i += 1;
@@ -175,13 +198,15 @@ template <class H> PRR_DEV void ref_rkf_h(const FrameParams &fp, const H &hk, Re
         V4<float> kx5 = v4scl(h, z5u), ku5 = v4scl(h, hk.geod(z5x, z5u));
         _x = v4add(v4add(v4add(v4add(v4add(x, v4scl(K::K41, kx1)), v4scl(K::K42, kx2)), v4scl(K::K43, kx3)), v4scl(K::K44, kx4)), v4scl(K::K45, kx5));
         _u = v4add(v4add(v4add(v4add(v4add(u, v4scl(K::K41, ku1)), v4scl(K::K42, ku2)), v4scl(K::K43, ku3)), v4scl(K::K44, ku4)), v4scl(K::K45, ku5));
-        // The sixth stage (zero weight in _x, _u) and the error decide nothing in intersection mode, nor where they are
-        // known to leave an hmax step at hmax; a warp evaluates them when one of its lanes needs them.
-        bool quiet = intersect && i <= 10000;
-        if constexpr (H::kErrorBound) quiet = quiet || (bounded && h == hmax && hk.small_error(x, u, h));
+        // The sixth stage (zero weight in _x, _u) and the error decide nothing in intersection mode while the stage is
+        // finite (0 * NaN is NaN), nor where they are known to leave an hmax step at hmax.  Each ray decides for itself, so
+        // no outcome depends on a warp's other rays; nothing is known of a header's geodesic, which is always evaluated.
+        bool quiet = false;
+        if constexpr (H::kErrorBound)
+            quiet = intersect && i <= 10000 ? hk.finite_stage(x, u, h) : bounded && h == hmax && hk.small_error(x, u, h);
         float maxerr = 0.0f;
         _h = hmax;
-        if (__any_sync(__activemask(), !quiet)) {
+        if (!quiet) {
             V4<float> z6x = v4add(v4add(v4add(v4add(v4add(x, v4scl(K::A61, kx1)), v4scl(K::A62, kx2)), v4scl(K::A63, kx3)), v4scl(K::A64, kx4)), v4scl(K::A65, kx5));
             V4<float> z6u = v4add(v4add(v4add(v4add(v4add(u, v4scl(K::A61, kx1)), v4scl(K::A62, ku2)), v4scl(K::A63, ku3)), v4scl(K::A64, ku4)), v4scl(K::A65, ku5));
             V4<float> kx6 = v4scl(h, z6u), ku6 = v4scl(h, hk.geod(z6x, z6u));
@@ -237,9 +262,5 @@ template <class H> PRR_DEV void ref_euler_h(const FrameParams &fp, const H &hk, 
     }
     R.result = PRR_RESULT_INFINITE_GEO;
 }
-
-PRR_DEV void ref_init(const FrameParams &fp, int x, int y, int s, RefRay &R) { ref_init_h(fp, BuiltinHooks{fp}, x, y, s, R); }
-PRR_DEV void ref_rkf(const FrameParams &fp, RefRay &R) { ref_rkf_h(fp, BuiltinHooks{fp}, R); }
-PRR_DEV void ref_euler(const FrameParams &fp, RefRay &R) { ref_euler_h(fp, BuiltinHooks{fp}, R); }
 
 }  // namespace prr

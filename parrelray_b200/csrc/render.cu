@@ -417,7 +417,7 @@ prr_status run_plan(prr_ctx *ctx, const RenderPlan &plan, uint8_t *d_rgb8, float
                 PRR_CK(ctx, (cudaError_t)tr(&p, d_fp, f, nr, ctx->rays.p, nullptr, rgb, counters, st));
                 launches += 3;
             } else if (plan.mode == PRR_MODE_REFERENCE) {
-                PRR_CK(ctx, launch_ref_trace(d_fp, f, nr, nullptr, rgb, counters, st));
+                PRR_CK(ctx, launch_ref_trace(p, d_fp, f, nr, nullptr, rgb, counters, st));
                 launches++;
             } else {
                 PlainBuffers b{ctx->rays.p, rgb};
@@ -512,7 +512,7 @@ prr_status trace_plan(prr_ctx *ctx, const RenderPlan &plan, float *h_state, doub
         PRR_CK(ctx, (cudaError_t)tr(&p, d_fp, 0, nr, ctx->rays.p, (float *)ctx->state.p, rgb, counters, st));
         ctx->last_launches = 3;
     } else if (plan.mode == PRR_MODE_REFERENCE) {
-        PRR_CK(ctx, launch_ref_trace(d_fp, 0, nr, (float *)ctx->state.p, rgb, counters, st));
+        PRR_CK(ctx, launch_ref_trace(p, d_fp, 0, nr, (float *)ctx->state.p, rgb, counters, st));
         ctx->last_launches = 1;
     } else if (ctx->schedule == PRR_SCHED_PLAIN && !h_state64) {
         if ((s = alloc(ctx, ctx->rays, (size_t)nr * plain_ray_record_bytes(), "ray records")) != PRR_OK) return s;
