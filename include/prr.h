@@ -474,6 +474,9 @@ prr_status prr_measure_peak(prr_ctx *ctx, double *fp32_tflops, double *fp64_tflo
  * inputs x[i] (1 <= n <= 2^20), out[4i .. 4i+3] = FP64 1/x, FP64 1/sqrt(x),
  * FP32 1/(float)x, FP32 1/sqrt((float)x) (the FP32 values widened). */
 prr_status prr_check_recip(prr_ctx *ctx, const double *x, int n, double *out);
+/* The same for the FP64 forms of the Hamiltonian FP64 renderer and the
+ * adjoint's reverse sweep: out[2i], out[2i+1] = 1/x, 1/sqrt(x). */
+prr_status prr_check_recip_h3(prr_ctx *ctx, const double *x, int n, double *out);
 
 /* ---- input decks (replaces main/io.h:21-58 readParams, the getters of
  *      main/Parameters.cpp:20-44, checkFrame prr.cpp:139-153, createScene

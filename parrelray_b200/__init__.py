@@ -118,6 +118,13 @@ class Context:
         self._check(self.lib.prr_check_recip(self.h, xs.ctypes.data_as(abi._dp), xs.size, out.ctypes.data_as(abi._dp)))
         return out
 
+    def check_recip_h3(self, x: np.ndarray) -> np.ndarray:
+        """prr_check_recip_h3: (n, 2) float64 of the third-order FP64 1/x and 1/sqrt(x)."""
+        xs = np.ascontiguousarray(x, dtype=np.float64).ravel()
+        out = np.empty((xs.size, 2), dtype=np.float64)
+        self._check(self.lib.prr_check_recip_h3(self.h, xs.ctypes.data_as(abi._dp), xs.size, out.ctypes.data_as(abi._dp)))
+        return out
+
     def render(self, frames, want_float: bool = False, out8: np.ndarray | None = None):
         """Renders one or more frames; returns (list of uint8 (h, w, 3)
         images, list of float32 images or None, Stats).  `out8` may supply

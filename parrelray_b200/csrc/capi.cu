@@ -411,21 +411,32 @@ prr_status prr_measure_peak(prr_ctx *ctx, double *fp32_tflops, double *fp64_tflo
     return PRR_OK;
 }
 
-prr_status prr_check_recip(prr_ctx *ctx, const double *x, int n, double *out)
+static prr_status check_recip(prr_ctx *ctx, const char *name, const double *x, int n, double *out, int per_input,
+                              cudaError_t (*launch)(const double *, int, double *, cudaStream_t))
 {
     if (!ctx) return PRR_ERR_INVALID;
     if (!x || !out || n < 1 || n > (1 << 20)) {
-        ctx->err = "prr_check_recip: needs 1..2^20 inputs and an output of 4 doubles per input";
+        ctx->err = std::string(name) + ": needs 1..2^20 inputs and an output of " + std::to_string(per_input) + " doubles per input";
         return PRR_ERR_INVALID;
     }
     PRR_CK(ctx, cudaSetDevice(ctx->device));
-    if (ensure_or_release(ctx, ctx->scratch, (size_t)n * 5 * sizeof(double)) != PRR_OK) return PRR_ERR_NOMEM;
+    if (ensure_or_release(ctx, ctx->scratch, (size_t)n * (1 + per_input) * sizeof(double)) != PRR_OK) return PRR_ERR_NOMEM;
     double *d_x = (double *)ctx->scratch.p, *d_out = d_x + n;
     PRR_CK(ctx, cudaMemcpyAsync(d_x, x, (size_t)n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-    PRR_CK(ctx, launch_check_recip(d_x, n, d_out, ctx->stream));
-    PRR_CK(ctx, cudaMemcpyAsync(out, d_out, (size_t)n * 4 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    PRR_CK(ctx, launch(d_x, n, d_out, ctx->stream));
+    PRR_CK(ctx, cudaMemcpyAsync(out, d_out, (size_t)n * per_input * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     PRR_CK(ctx, cudaStreamSynchronize(ctx->stream));
     return PRR_OK;
+}
+
+prr_status prr_check_recip(prr_ctx *ctx, const double *x, int n, double *out)
+{
+    return check_recip(ctx, "prr_check_recip", x, n, out, 4, launch_check_recip);
+}
+
+prr_status prr_check_recip_h3(prr_ctx *ctx, const double *x, int n, double *out)
+{
+    return check_recip(ctx, "prr_check_recip_h3", x, n, out, 2, launch_check_recip_h3);
 }
 
 }  // extern "C"

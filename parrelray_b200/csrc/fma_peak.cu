@@ -43,17 +43,30 @@ __global__ void k_check_recip(const double *x, int n, double *out)
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double v = x[i];
-    // of the two FP64 forms in use, the value with the larger residual
-    const double x1 = frcp<double>(v), x3 = h3_rcp(v), y1 = frsqrt<double>(v), y3 = h3_rsqrt(v);
-    out[4 * i] = fabs(fma(-v, x3, 1.0)) > fabs(fma(-v, x1, 1.0)) ? x3 : x1;
-    out[4 * i + 1] = fabs(fma(-v * y3, y3, 1.0)) > fabs(fma(-v * y1, y1, 1.0)) ? y3 : y1;
+    out[4 * i] = frcp<double>(v);
+    out[4 * i + 1] = frsqrt<double>(v);
     out[4 * i + 2] = (double)frcp<float>((float)v);
     out[4 * i + 3] = (double)frsqrt<float>((float)v);
+}
+
+// The FP64 renderer's third-order forms (h3_rcp, h3_rsqrt) on x[i]: out[2i], out[2i+1] = 1/x, 1/sqrt(x).
+__global__ void k_check_recip_h3(const double *x, int n, double *out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    out[2 * i] = h3_rcp(x[i]);
+    out[2 * i + 1] = h3_rsqrt(x[i]);
 }
 
 cudaError_t launch_check_recip(const double *x, int n, double *out, cudaStream_t st)
 {
     k_check_recip<<<(n + 255) / 256, 256, 0, st>>>(x, n, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_check_recip_h3(const double *x, int n, double *out, cudaStream_t st)
+{
+    k_check_recip_h3<<<(n + 255) / 256, 256, 0, st>>>(x, n, out);
     return cudaGetLastError();
 }
 

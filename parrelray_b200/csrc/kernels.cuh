@@ -138,7 +138,8 @@ int adjoint_window(size_t budget, int threads, int max_steps, int precision);
 // fma_peak.cu
 cudaError_t launch_fma_peak(float *sink, int blocks, int threads, int iters, cudaStream_t st);
 cudaError_t launch_dfma_peak(double *sink, int blocks, int threads, int iters, cudaStream_t st);
-// fma_peak.cu: frcp/frsqrt (FP64 and FP32) on n inputs, 4 outputs each
+// fma_peak.cu: frcp/frsqrt (FP64 and FP32) on n inputs, 4 outputs each; the third-order FP64 forms, 2 each
 cudaError_t launch_check_recip(const double *x, int n, double *out, cudaStream_t st);
+cudaError_t launch_check_recip_h3(const double *x, int n, double *out, cudaStream_t st);
 
 }  // namespace prr
