@@ -246,7 +246,8 @@ typedef struct prr_stats {
 /* Launch shape of the persistent scheduler. */
 typedef struct prr_launch_config {
     int32_t block_size;          /* threads per CTA (multiple of 32) */
-    int32_t blocks_per_sm;       /* resident CTAs per SM requested */
+    int32_t blocks_per_sm;       /* resident CTAs per SM, at most (0: the occupancy limit): a launch with
+                                    fewer work items than lanes starts only as many as find work */
     int32_t compaction_interval; /* attempts between warp refills */
     int32_t rays_per_thread;     /* FP32 renders: pixels in flight per thread, 1 or 2 (2: the two
                                     rays' stages share paired FP32 instructions); results do not
@@ -399,7 +400,7 @@ prr_status prr_graph_create(prr_ctx *ctx, const prr_frame_desc *frames, int n, u
 prr_status prr_graph_set_frames(prr_graph *g, const prr_frame_desc *frames, int n);
 prr_status prr_graph_launch(prr_graph *g, void *stream);
 prr_status prr_graph_stats(prr_graph *g, prr_stats *stats);
-/* The launch shape recorded in the graph (blocks_per_sm resolved). */
+/* The launch shape recorded in the graph (blocks_per_sm resolved; the most CTAs per SM a launch may start). */
 prr_status prr_graph_get_launch_config(const prr_graph *g, prr_launch_config *cfg);
 void prr_graph_destroy(prr_graph *g);
 

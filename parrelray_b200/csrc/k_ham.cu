@@ -905,7 +905,9 @@ cudaError_t launch_ham(const PersistentArgs &args, int precision, bool split, in
     if (grid < 1) grid = 1;
     // Below one full warp per scheduler, one warp on each with as many lanes as there is work: a warp leaves the quick
     // loop when one of its lanes has to, so fewer lanes share fewer detours.  Medians: 96x54 frame 2.04 -> 1.80 ms,
-    // 60x33 1.82 -> 1.45, 180x101 2.65 -> 2.32, FP64 60x33 3.03 -> 2.47, 100x56 3.38 -> 3.41, 180x101 4.45 -> 3.90.
+    // 60x33 1.82 -> 1.45, 180x101 2.65 -> 2.32, FP64 60x33 3.03 -> 2.47, 100x56 3.38 -> 3.41, 180x101 4.45 -> 3.90.  (CTAs of 96
+    // threads leave a scheduler without a warp and some items waiting, yet two of them per SM are slower: 60x33 1.39 against
+    // 1.58, FP64 2.34 and 2.84; for 160 to 256 threads lanes for all 5 to 8 warps gain and lose up to a tenth by size.)
     const long long schedulers = 4ll * nsm, per = (a.total_pixels + schedulers - 1) / schedulers;
     if (per < 32 && blocks_per_sm * block >= 128) {
         a.lanes = per > 1 ? (int)per : 1;
