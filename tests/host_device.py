@@ -19,6 +19,8 @@ SHIM = r"""
 #include <cuda_runtime.h>
 using std::acos; using std::atan2; using std::fabs; using std::floor; using std::fmax; using std::fmin; using std::isnan;
 using std::max; using std::min; using std::sqrt;
+#undef __noinline__
+#define __noinline__  // a macro of nvcc's
 inline double __fma_rn(double a, double b, double c) { return std::fma(a, b, c); }
 inline float __fmaf_rn(float a, float b, float c) { return std::fma(a, b, c); }
 inline float __fmul_rn(float a, float b) { return a * b; }
