@@ -686,8 +686,10 @@ extern "C" prr_status prr_adjoint(prr_ctx *ctx, const prr_frame_desc *frame, con
     int threads = (int)std::min<long long>((long long)ctx->nsm * adjoint_blocks_per_sm(prec) * 128, (nrays + 127) / 128 * 128);
     // The states of a window and the checkpoints of the earlier ones are sized together: a quarter of the free memory at
     // most (or what the context holds already), then, where that cannot be had, the smallest pair, then fewer threads.
-    size_t spare = spare_bytes(ctx->adj_states.cap + ctx->adj_ckpt.cap);
+    size_t spare = ctx->adj_states.cap + ctx->adj_ckpt.cap;
+    if (adjoint_window(spare, threads, d.max_steps, prec) < adjoint_window(SIZE_MAX, threads, d.max_steps, prec)) spare = spare_bytes(spare);
     int cap = 0, max_ckpt = 0;
+    bool tight = false;
     while (true) {
         cap = ctx->adj_window ? ctx->adj_window : adjoint_window(spare, threads, d.max_steps, prec);
         max_ckpt = d.max_steps / cap + 2;
@@ -697,7 +699,7 @@ extern "C" prr_status prr_adjoint(prr_ctx *ctx, const prr_frame_desc *frame, con
         cudaGetLastError();  // the failed allocation's
         ctx->adj_states.release();
         ctx->adj_ckpt.release();
-        if (spare) spare = 0;
+        if (!tight) { spare = 0; tight = true; }
         else if (threads > 128) threads = std::max(128, threads / 256 * 128);
         else { ctx->err = "out of device memory for adjoint states"; return PRR_ERR_NOMEM; }
     }
