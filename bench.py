@@ -80,6 +80,8 @@ F_ATTEMPT = 6 * FLOPS_GEOD_KERR + FLOPS_STAGES
 # executes 684 FLOP per attempt (most attempts leave out the sixth stage and the error estimate); k_pair (the
 # (x, u) contraction, the form F_ATTEMPT counts) 1,459.
 NCU_FLOP_PER_ATTEMPT = {"k_ham": 684.0, "k_pair": 1459.0}
+# The same count of FP64 operations of k_ham<double> (DFMA 2 FLOP, DMUL and DADD 1).
+NCU_FP64_FLOP_PER_ATTEMPT = 741.0
 NCU_FLOP_RULE = ("FP32 FLOP executed, from ncu sass_thread_inst_executed_op_{ffma,fmul,fadd}{,2}: FFMA 2, FFMA2 4, "
                  "FMUL/FADD 1, FMUL2/FADD2 2, per attempt")
 # DRAM bytes of one launch of the tracing kernel (ncu, 960x540 copy of the headline frame)
@@ -770,10 +772,11 @@ def bench_accuracy(ctx, frame, fp64_peak, n_oracle_rays: int = 4096) -> dict:
     res = {"pixels_within_1_255_of_fp64_gpu": float(np.mean(d <= 1)), "max_abs_diff_255": int(d.max()),
            "fp64_ms": s64.kernel_ms}
     if s64.trace_ms > 0:
-        # the FP64 render's tracing kernel against the measured FP64 FMA peak (same F_attempt)
-        a64 = s64.attempts * F_ATTEMPT / (s64.trace_ms * 1e-3) / 1e12
+        # the FP64 render's tracing kernel against the measured FP64 FMA peak, by the operations it executes
+        a64 = s64.attempts * NCU_FP64_FLOP_PER_ATTEMPT / (s64.trace_ms * 1e-3) / 1e12
         res["fp64_roofline"] = {"achieved": a64, "peak": fp64_peak, "unit": "TFLOP/s", "frac": a64 / fp64_peak,
-                                "attempts": int(s64.attempts)}
+                                "attempts": int(s64.attempts),
+                                "flop_per_attempt": NCU_FP64_FLOP_PER_ATTEMPT, "what": "executed FP64 FLOP (ncu), k_ham<double>"}
     try:
         sys.path.insert(0, str(REPO / "tests"))
         from oracles import Oracle, kerr_criticality

@@ -1,6 +1,6 @@
-// k_ham.cu - the FP32 renderer of PHYSICAL frames (one pixel in flight per
-// thread) with the geodesic in Hamiltonian form; with SPLIT, the FP32 pass of a
-// split-precision render; with EMIS, plasma emission along the rays.
+// k_ham.cu - the FP32 and FP64 renderers of PHYSICAL frames (one ray in flight
+// per thread) with the geodesic in Hamiltonian form; with SPLIT, the FP32 pass of
+// a split-precision render; with EMIS, plasma emission along the rays.
 //
 // The geodesics of the Kerr-Schild metric g = eta + f l(x)l are integrated
 // as the canonical system of H = 1/2 g^{ab} p_a p_b with the inverse metric

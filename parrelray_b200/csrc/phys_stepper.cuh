@@ -135,8 +135,9 @@ template <class T> PRR_DEV bool sphere_d(const DevSphere &S, T px, T py, T pz, T
 
 // True when the point p is too far from sphere S for Sphere::intersects to
 // accept it with any window h <= hmax: a hit needs the distance to the
-// centre D to satisfy D^2 <= ((sqrt(hmax) + R)/2)^2 + R^2 (S.far2 holds
-// that bound with a rounding margin), so skipping the test changes nothing.
+// centre D to satisfy D^2 <= R^2 + hmax/3 (S.far2 holds that bound with a
+// rounding margin, or a wider one where the first step may exceed hmax:
+// render.cu:build_plan), so skipping the test changes nothing.
 template <class T> PRR_DEV bool sphere_far(const DevSphere &S, T px, T py, T pz)
 {
     T dx = px - (T)S.cx, dy = py - (T)S.cy, dz = pz - (T)S.cz;
