@@ -8,10 +8,9 @@
 // error are evaluated only where they can decide something, and the sphere
 // test only near a sphere (ref_stepper.cuh): 1920x1080x4 Kerr frame at eps
 // 1e-3 813 -> 628 ms, 320x180x4 64 -> 51 ms, 320x180 Schwarzschild 13.8 ->
-// 11.3 ms, the same bits.  The Kerr geodesic has a kernel of its own: with
-// both geodesics in each of the six stages 320x180 with three spheres took
-// 40.1 ms (Schwarzschild 37.6, without spheres 6.0, Kerr 960x540x4 164), and
-// takes 33.7 (35.2, 5.6, 148) with one.
+// 11.3 ms, the same bits.  The Kerr geodesic has a kernel of its own: with both
+// geodesics at each of the six stages these frames took 628, 51 and 11.3
+// ms, with one they take 580, 43 and 10.7.
 #include "kernels.cuh"
 #include "ref_stepper.cuh"
 
@@ -70,8 +69,9 @@ cudaError_t launch_ref_trace(const FrameParams &fp, const FrameParams *d_fp, int
 {
     if (nrays <= 0) return cudaSuccess;
     // a warp leaves when its longest ray does: one-warp CTAs free their slots at once, which a frame of about a wave
-    // likes (320x180: 11.3 ms against 11.8 with four warps), and a large one not (1920x1080x4: 636 and 628), nor one
-    // whose eps is so tight that rays take up to 10^6 attempts (96x54 at eps 1e-6: 4.78 s against 4.56)
+    // likes (320x180 Schwarzschild 10.7 ms against 11.3 with four warps, 640x360 Kerr 43.8 and 44.4), and a large one not
+    // (1920x1080x4: 582 and 580), nor one whose eps is so tight that rays take up to 10^6 attempts (96x54 at eps 1e-6: 4.78 s
+    // against 4.56)
     const int block = ref_bounded(fp) && nrays <= (1 << 19) ? 32 : 128;
     long long grid = (nrays + block - 1) / block;
     auto k = fp.metric == PRR_METRIC_KERR ? k_ref_trace<true> : k_ref_trace<false>;
