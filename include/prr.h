@@ -335,7 +335,7 @@ prr_status prr_trace_rays_f64(prr_ctx *ctx, const prr_frame_desc *frame,
  * steps, 36 bytes each (72 with FP64 steps), and a checkpoint per earlier
  * window, whose steps are recomputed.  The window is 4096 steps (8.4 and
  * 11 GB) where that is at most a quarter of the free memory, and shorter
- * otherwise, down to under 1 GB; PRR_OPT_ADJOINT_WINDOW sets it.  The context
+ * otherwise (under 1 GB at max_steps 10000); PRR_OPT_ADJOINT_WINDOW sets it.  The context
  * keeps these buffers for its next gradient and gives them back when it runs
  * short of memory itself, or in prr_destroy. */
 prr_status prr_adjoint(prr_ctx *ctx, const prr_frame_desc *frame, const float *dL_dimage, int sphere_index,
